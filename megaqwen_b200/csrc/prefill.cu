@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "mma_attention.cuh"
 #include "sk_chain.cuh"
 #include "tc_attention.cuh"
 #include "tc_gemm2.cuh"
@@ -147,216 +148,17 @@ __global__ void __launch_bounds__(256) k_pf_qknorm_rope(bf16* __restrict__ qkv, 
     }
 }
 
-// ---------------------------------------------------------------- causal GQA attention (prefill)
-// QK^T and PV run on mma.sync m16n8k16 (bf16 in, fp32 accumulate) with an online softmax in
-// registers; probabilities are rounded to bf16 before the PV product and the row sum uses the
-// unrounded values.
-// Causal attention of the prompt.  One CTA per (query head, 64-query tile).  Under the causal
-// mask the last query tile of a prompt has sixteen times the work of the first, and the pass
-// is as long as its longest CTA, so the key tiles of a query tile are dealt out to FA_NG
-// groups of four warps that walk them in parallel (group g takes key tiles g, g + FA_NG, ..)
-// and are merged through shared memory at the end; the grid is ordered longest query tile
-// first.  Each group streams its K/V tiles through its own two-stage ring of padded rows
-// (16-byte cp.async, the next tile in flight while this one is multiplied).
-constexpr int FA_BQ = 64, FA_BK = 64, FA_LD = D + 8, FA_NG = 2, FA_THREADS = FA_NG * 128;
-constexpr int FA_TILE_ELEMS = FA_BK * FA_LD;                                  // one K or V tile
-constexpr size_t FA_SMEM = (size_t)(FA_BQ * FA_LD + FA_NG * 2 * 2 * FA_TILE_ELEMS) * 2;
-
-__device__ __forceinline__ void group_barrier(int group) {
-    asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory");
-}
-
-__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const bf16* p) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
-}
-__device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const bf16* p) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
-}
-__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
+// ---------------------------------------------------------------- causal GQA attention of a prompt below 128 rows
 __global__ void __launch_bounds__(FA_THREADS, 1) k_pf_attention(const bf16* __restrict__ qkv, const bf16* __restrict__ k_cache,
                                                                const bf16* __restrict__ v_cache, bf16* __restrict__ out, int S, int pos0,
                                                                int layer, int max_seq) {
     pdl_trigger();   // the next grid may be scheduled already (it waits the same way)
     pdl_wait();      // launched with programmatic stream serialisation: the preceding grid has completed
     extern __shared__ __align__(16) uint8_t fa_smem[];
-    bf16* sq = reinterpret_cast<bf16*>(fa_smem);                    // [64][FA_LD]
-    bf16* ring = sq + FA_BQ * FA_LD;                                // [FA_NG][2 stages][K tile | V tile]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int grp = warp >> 2, wq = warp & 3, gtid = tid & 127;
-    const int head = blockIdx.x, g = head / (NQ / NKV);
+    const int head = blockIdx.x;
+    const size_t plane = (size_t)(layer * NKV + head / (NQ / NKV)) * max_seq * D;
     const int q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * FA_BQ;  // longest query tiles are dispatched first
-    const bf16* kbase = k_cache + ((size_t)(layer * NKV + g) * max_seq) * D;
-    const bf16* vbase = v_cache + ((size_t)(layer * NKV + g) * max_seq) * D;
-    bf16* gring = ring + (size_t)grp * 4 * FA_TILE_ELEMS;
-
-    const int kv_end = min(pos0 + S, pos0 + q0 + FA_BQ);     // exclusive bound of keys any row of the tile may see
-    const int ntiles = (kv_end + FA_BK - 1) / FA_BK;
-    auto load_tile = [&](int t, int stage) {
-        bf16* sk = gring + (size_t)stage * 2 * FA_TILE_ELEMS;
-        bf16* sv = sk + FA_TILE_ELEMS;
-        const int p0 = t * FA_BK;
-        for (int c = gtid; c < FA_BK * (D / 8); c += 128) {
-            const int r = c / (D / 8), cc = c % (D / 8);
-            const bool ok = p0 + r < kv_end;
-            const size_t off = (size_t)(ok ? p0 + r : 0) * D + cc * 8;
-            cp_async16_zfill(sk + r * FA_LD + cc * 8, kbase + off, ok);
-            cp_async16_zfill(sv + r * FA_LD + cc * 8, vbase + off, ok);
-        }
-    };
-    if (grp < ntiles) load_tile(grp, 0);
-    cp_async_commit();
-
-    // Q tile -> shared (rows past S are zero)
-    for (int c = tid; c < FA_BQ * (D / 8); c += FA_THREADS) {
-        const int r = c / (D / 8), cc = c % (D / 8);
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (q0 + r < S) v = *reinterpret_cast<const uint4*>(qkv + (size_t)(q0 + r) * QKV + head * D + cc * 8);
-        *reinterpret_cast<uint4*>(sq + r * FA_LD + cc * 8) = v;
-    }
-    __syncthreads();
-    uint32_t qf[8][4];
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk)
-        ldsm_x4(qf[kk], sq + (wq * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * FA_LD + kk * 16 + (lane >> 4) * 8);
-
-    float o[16][4];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
-    float m_run[2] = {-1e30f, -1e30f}, l_run[2] = {0.f, 0.f};
-    // scores are kept in the log2 domain (scale * log2(e) folded in) so that the softmax uses
-    // the single-instruction exp2 instead of expf; the probabilities are the same numbers
-    const float scale = 0.08838834764831845f * 1.4426950408889634f;
-    const int row_a = pos0 + q0 + wq * 16 + (lane >> 2);   // absolute position of this thread's first row; second is +8
-
-    int it = 0;
-    for (int t = grp; t < ntiles; t += FA_NG, ++it) {
-        // the other stage was consumed in the previous iteration (barrier at its end): request the next tile
-        if (t + FA_NG < ntiles) load_tile(t + FA_NG, (it + 1) & 1);
-        cp_async_commit();
-        cp_async_wait<1>();          // this thread's copies of tile t have landed
-        group_barrier(grp);          // .. and everybody's in the group
-        const bf16* sk = gring + (size_t)(it & 1) * 2 * FA_TILE_ELEMS;
-        const bf16* sv = sk + FA_TILE_ELEMS;
-        const int p0 = t * FA_BK;
-
-        float sacc[8][4];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) { sacc[i][0] = sacc[i][1] = sacc[i][2] = sacc[i][3] = 0.f; }
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-#pragma unroll
-            for (int np = 0; np < 4; ++np) {   // pairs of 8-key tiles
-                uint32_t kf[4];
-                ldsm_x4(kf, sk + (np * 16 + (lane & 7) + (lane >> 4) * 8) * FA_LD + kk * 16 + ((lane >> 3) & 1) * 8);
-                mma_bf16_16816(sacc[2 * np], qf[kk], kf[0], kf[1]);
-                mma_bf16_16816(sacc[2 * np + 1], qf[kk], kf[2], kf[3]);
-            }
-        }
-        // scale, causal mask, online softmax
-        float mx[2] = {-1e30f, -1e30f};
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int key = p0 + nt * 8 + (lane & 3) * 2 + (e & 1);
-                const int rowp = row_a + (e >> 1) * 8;
-                const float sv_ = (key <= rowp) ? sacc[nt][e] * scale : -1e30f;
-                sacc[nt][e] = sv_;
-                mx[e >> 1] = fmaxf(mx[e >> 1], sv_);
-            }
-        }
-        float corr[2];
-#pragma unroll
-        for (int h2 = 0; h2 < 2; ++h2) {
-            mx[h2] = fmaxf(mx[h2], __shfl_xor_sync(0xffffffffu, mx[h2], 1));
-            mx[h2] = fmaxf(mx[h2], __shfl_xor_sync(0xffffffffu, mx[h2], 2));
-            const float m_new = fmaxf(m_run[h2], mx[h2]);
-            corr[h2] = fast_exp2(m_run[h2] - m_new);
-            m_run[h2] = m_new;
-        }
-        float rs[2] = {0.f, 0.f};
-        uint32_t pf[4][4];
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-            float pe[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                pe[e] = (sacc[nt][e] <= -1e29f) ? 0.f : fast_exp2(sacc[nt][e] - m_run[e >> 1]);
-                rs[e >> 1] += pe[e];
-            }
-            pf[nt >> 1][(nt & 1) * 2 + 0] = pack_bf16x2(pe[0], pe[1]);
-            pf[nt >> 1][(nt & 1) * 2 + 1] = pack_bf16x2(pe[2], pe[3]);
-        }
-#pragma unroll
-        for (int h2 = 0; h2 < 2; ++h2) {
-            rs[h2] += __shfl_xor_sync(0xffffffffu, rs[h2], 1);
-            rs[h2] += __shfl_xor_sync(0xffffffffu, rs[h2], 2);
-            l_run[h2] = l_run[h2] * corr[h2] + rs[h2];
-        }
-#pragma unroll
-        for (int dt = 0; dt < 16; ++dt) { o[dt][0] *= corr[0]; o[dt][1] *= corr[0]; o[dt][2] *= corr[1]; o[dt][3] *= corr[1]; }
-        // O += P V
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {          // 16 keys per step
-#pragma unroll
-            for (int dp = 0; dp < 8; ++dp) {   // pairs of 8-wide output tiles
-                uint32_t vf[4];
-                ldsm_x4_t(vf, sv + (j * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * FA_LD + dp * 16 + (lane >> 4) * 8);
-                mma_bf16_16816(o[2 * dp], pf[j], vf[0], vf[1]);
-                mma_bf16_16816(o[2 * dp + 1], pf[j], vf[2], vf[3]);
-            }
-        }
-        group_barrier(grp);          // the stage may be overwritten by the next iteration's request
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    // merge the groups: groups 1.. leave (m, l, O) of every thread in the ring, group 0 combines
-    float* xch = reinterpret_cast<float*>(ring);        // [FA_NG - 1][128 threads][68]
-    if (grp > 0) {
-        float* mine = xch + ((size_t)(grp - 1) * 128 + gtid) * 68;
-        mine[0] = m_run[0]; mine[1] = m_run[1]; mine[2] = l_run[0]; mine[3] = l_run[1];
-#pragma unroll
-        for (int dt = 0; dt < 16; ++dt) *reinterpret_cast<float4*>(mine + 4 + dt * 4) = make_float4(o[dt][0], o[dt][1], o[dt][2], o[dt][3]);
-    }
-    __syncthreads();
-    if (grp > 0) return;
-#pragma unroll
-    for (int og = 1; og < FA_NG; ++og) {
-        const float* oth = xch + ((size_t)(og - 1) * 128 + gtid) * 68;
-        float f_me[2], f_ot[2];
-#pragma unroll
-        for (int h2 = 0; h2 < 2; ++h2) {
-            const float mo = oth[h2], mn = fmaxf(m_run[h2], mo);
-            f_me[h2] = fast_exp2(m_run[h2] - mn);
-            f_ot[h2] = fast_exp2(mo - mn);
-            l_run[h2] = l_run[h2] * f_me[h2] + oth[2 + h2] * f_ot[h2];
-            m_run[h2] = mn;
-        }
-#pragma unroll
-        for (int dt = 0; dt < 16; ++dt) {
-            const float4 ov = *reinterpret_cast<const float4*>(oth + 4 + dt * 4);
-            o[dt][0] = o[dt][0] * f_me[0] + ov.x * f_ot[0];
-            o[dt][1] = o[dt][1] * f_me[0] + ov.y * f_ot[0];
-            o[dt][2] = o[dt][2] * f_me[1] + ov.z * f_ot[1];
-            o[dt][3] = o[dt][3] * f_me[1] + ov.w * f_ot[1];
-        }
-    }
-    // normalise and store
-    const int r_lo = q0 + wq * 16 + (lane >> 2), r_hi = r_lo + 8;
-    const float inv0 = 1.0f / l_run[0], inv1 = 1.0f / l_run[1];
-#pragma unroll
-    for (int dt = 0; dt < 16; ++dt) {
-        const int col = head * D + dt * 8 + (lane & 3) * 2;
-        if (r_lo < S) *reinterpret_cast<uint32_t*>(out + (size_t)r_lo * QSZ + col) = pack_bf16x2(o[dt][0] * inv0, o[dt][1] * inv0);
-        if (r_hi < S) *reinterpret_cast<uint32_t*>(out + (size_t)r_hi * QSZ + col) = pack_bf16x2(o[dt][2] * inv1, o[dt][3] * inv1);
-    }
+    fa_tile(fa_smem, qkv, k_cache + plane, v_cache + plane, out, S, pos0, q0, head);
 }
 
 // ---------------------------------------------------------------- host side
@@ -793,7 +595,7 @@ static int prefill_impl(const MqModel* model, const MqDecodeBuffers* dbuf, const
                         int seq_len, int pos0, const bf16* audio, int audio_start, int audio_len, int* out_token, float* logits,
                         void* stream_v);
 
-// The chain of few rows: q|k|v (with everything up to the cache), and what follows the attention.
+// The chain of a batch's decode step: q|k|v (with everything up to the cache), and what follows the attention.
 static SkArgs sk_args(const MqModel* model, int rows, bf16* h, float* ssq, bf16* k_cache, bf16* v_cache, unsigned int* status) {
     SkArgs a = {};
     a.M = rows; a.h = h; a.ssq = ssq; a.status = status;
@@ -826,8 +628,8 @@ static int sk_rest(const MqModel* model, int l, SkArgs a, const bf16* attn, bf16
 //   gate|up 16.0 / 18.5  30.0 / 19.9  30.3 / 25.3  59.1 / 42.4   242 / 148
 //   o       14.5 / 18.3  14.7 / 18.5  14.6 / 19.4  29.2 / 22.2   131 / 76
 //   down    19.3 / 23.9  20.0 / 24.3  20.1 / 25.1  39.4 / 27.9   155 / 85
-// Below, tiles are as wide as leaves one round of CTAs.  Prompt of 129 / 256 / 384 / 640 / 900 / 1000 rows with 128-wide tiles
-// everywhere and the split of K from 512 rows on: 1.97 / 2.04 / 2.08 / 2.19 / 2.65 / 2.69 ms, now 1.62 / 1.68 / 1.76 / 2.12 / 2.30 / 2.33.
+// Below, tiles are as wide as leaves one round of CTAs.  Prompt of 2 / 23 / 128 / 256 / 384 / 640 / 900 / 1024 rows with 128-wide tiles
+// everywhere: 1.76 / 1.82 / 2.00 / 2.03 / 2.10 / 2.22 / 2.72 / 2.41 ms, now 1.67 / 1.71 / 1.86 / 1.93 / 2.00 / 2.12 / 2.30 / 2.33.
 static int pf_qkv(const MqModel* model, int l, const bf16* x, bf16* qkv, int rows, Heads hd, unsigned int* status, cudaStream_t stream) {
     const MqLayerWeights& w = model->layers[l];
     const bf16 *q = (const bf16*)w.q_proj, *k = (const bf16*)w.k_proj, *v = (const bf16*)w.v_proj;
@@ -896,7 +698,7 @@ static int prefill_impl(const MqModel* model, const MqDecodeBuffers* dbuf, const
     // From 128 prompt rows on the attention runs on tcgen05, its K and V tiles straight from the cache.  The V map
     // is a stack of (layer, kv head) planes that end at the prompt's last key: what the cache holds beyond it
     // (possibly not even numbers) is multiplied by probabilities of zero and must read as zero.
-    const bool few = S <= SK_MAX_ROWS && dbuf->attn_partials != nullptr, use_tc = !few || S >= TA_BQ;
+    const bool use_tc = S >= TA_BQ;
     CUtensorMap map_q, map_k, map_v;
     if (use_tc) {
         int mrc = get_map(qkv, (uint64_t)S, (uint64_t)D, (uint64_t)QKV, TA_BQ, &map_q, (uint64_t)NQ, (uint64_t)D);
@@ -909,41 +711,15 @@ static int prefill_impl(const MqModel* model, const MqDecodeBuffers* dbuf, const
         if (mrc != MQ_OK) return mrc;
     }
     int rc;
-    // Up to 128 rows: the cluster chain, its row sums in the decode path's scratch (a caller without that scratch takes the
-    // tiles below, whose sums do not depend on the number of rows).
-    if (few) {
-        SkArgs a = sk_args(model, S, h, dbuf->attn_partials, (bf16*)dbuf->k_cache, (bf16*)dbuf->v_cache, status);
-        a.pos0 = pos0;
-        launch_pdl(k_sk_embed, dim3(S), dim3(128), 0, stream, ids, (const bf16*)model->embed, h, a.ssq, model->vocab_size, status, audio, audio_start, audio_len);
-        for (int l = 0; l < model->num_layers; ++l) {
-            rc = sk_qkv(model, l, a, qkv, stream);
-            if (rc) return rc;
-            if (use_tc) {
-                rc = launch_attention_tc<2, 0, 2>(NQ, map_q, map_k, map_v, map_q, map_k,
-                                                  {attn, QSZ, D, S, pos0, NQ / NKV, l * NKV, 8, 0, 0.08838834764831845f * 1.4426950408889634f, nullptr, status},
-                                                  stream);
-                if (rc) return rc;
-            } else {
-                launch_pdl(k_pf_attention, dim3(dim3(NQ, (S + FA_BQ - 1) / FA_BQ)), dim3(FA_THREADS), fa_smem, stream, qkv, (const bf16*)dbuf->k_cache,
-                           (const bf16*)dbuf->v_cache, attn, S, pos0, l, model->max_seq_len);
-            }
-            rc = sk_rest(model, l, a, attn, act, stream);
-            if (rc) return rc;
-        }
-        launch_pdl(k_pf_copy_row, dim3(1), dim3(H / 8), 0, stream, h + (size_t)(S - 1) * H, (bf16*)dbuf->hidden);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return (int)e;
-        return launch_lmhead_only(model, dbuf, out_token, logits, stream);
-    }
     launch_pdl(k_pf_embed, dim3(S), dim3(128), 0, stream, ids, (const bf16*)model->embed, h, model->vocab_size, status, audio,
                audio_start, audio_len);
-    // Up to 1024 rows the N = 1024 projections (O, down) split K over two CTAs per 128 x 128 tile (a caller without the decode path's
-    // scratch from 512 rows on: below, its sums do not depend on the number of rows):
+    // Between 512 and 1024 rows the N = 1024 projections (O, down) split K over two CTAs per 128 x 128 tile:
     // 64-wide tiles re-read the A operand sixteen times and are bound by L2 traffic.  The fp32 planes land in
     // the qkv buffer (free after attention; 2 x S x 1024 floats fill it exactly) and one kernel adds them to the
     // residual stream and applies the RMSNorm that follows (the next layer's input norm after the down projection).
     // Above 1024 and up to 2048 rows the same with 128 x 256 tiles (N = 256 instructions, half the A traffic per FLOP).
-    const bool splitk = (S >= 512 || dbuf->attn_partials != nullptr) && S <= 2048 && (size_t)pb->max_tokens * QKV * sizeof(bf16) >= (size_t)2 * S * H * sizeof(float);
+    // Below, sums over K stay whole.
+    const bool splitk = S >= 512 && S <= 2048 && (size_t)pb->max_tokens * QKV * sizeof(bf16) >= (size_t)2 * S * H * sizeof(float);
     const bool wide = splitk && S > 1024;
     float* part = reinterpret_cast<float*>(qkv);
     Heads heads = {};
@@ -954,10 +730,15 @@ static int prefill_impl(const MqModel* model, const MqDecodeBuffers* dbuf, const
             launch_pdl(k_pf_rmsnorm, dim3((S + 7) / 8), dim3(256), 0, stream, h, (const bf16*)w.input_layernorm, x, S);
         rc = pf_qkv(model, l, x, qkv, S, heads, status, stream);
         if (rc) return rc;
-        rc = launch_attention_tc<2, 0, 2>(NQ, map_q, map_k, map_v, map_q, map_k,
-                                          {attn, QSZ, D, S, pos0, NQ / NKV, l * NKV, 8, 0, 0.08838834764831845f * 1.4426950408889634f, nullptr, status},
-                                          stream);
-        if (rc) return rc;
+        if (use_tc) {
+            rc = launch_attention_tc<2, 0, 2>(NQ, map_q, map_k, map_v, map_q, map_k,
+                                              {attn, QSZ, D, S, pos0, NQ / NKV, l * NKV, 8, 0, 0.08838834764831845f * 1.4426950408889634f, nullptr, status},
+                                              stream);
+            if (rc) return rc;
+        } else {
+            launch_pdl(k_pf_attention, dim3(NQ, (S + FA_BQ - 1) / FA_BQ), dim3(FA_THREADS), fa_smem, stream, qkv, (const bf16*)dbuf->k_cache,
+                       (const bf16*)dbuf->v_cache, attn, S, pos0, l, model->max_seq_len);
+        }
         // N = 1024: with M <= 1024 a 128-wide tile gives at most 64 CTAs, 64-wide tiles double that
         if (splitk) {
             rc = wide ? launch_gemm<256, EPI_PARTIAL>(attn, QSZ, (const bf16*)w.o_proj, nullptr, (bf16*)part, nullptr, S, H, QSZ, H, status, stream,
@@ -1013,8 +794,8 @@ extern "C" int mq_launch_prefill_packed(const MqModel* model, const MqBatchBuffe
     bf16* h = (bf16*)pb->h; bf16* x = (bf16*)pb->x; bf16* qkv = (bf16*)pb->qkv; bf16* attn = (bf16*)pb->attn; bf16* act = (bf16*)pb->act;
     unsigned int* status = bb->status;
     const size_t seq_stride = (size_t)model->num_layers * NKV * model->max_seq_len * D;
-    // One attention kernel for all prompts whatever their lengths, the one that a single prompt takes in prefill_impl without scratch:
-    // same bits.  With mma.sync tiles of 64 queries in its place 64 x 1024 / 32 x ~384 rows took 108 / 17.7 ms, now 84.5 / 14.9.
+    // The attention that each prompt takes alone in prefill_impl: same bits.  With mma.sync tiles of 64 queries for prompts of 128 rows
+    // and more too, 64 x 1024 / 32 x ~384 rows took 108 / 17.7 ms, now 84.5 / 14.9.
     CUtensorMap map_q, map_k, map_v;
     const uint64_t planes = (uint64_t)B * model->num_layers * NKV;
     int rc = get_map(qkv, (uint64_t)T, (uint64_t)D, (uint64_t)QKV, TA_BQ, &map_q, (uint64_t)NQ, (uint64_t)D);
@@ -1024,6 +805,7 @@ extern "C" int mq_launch_prefill_packed(const MqModel* model, const MqBatchBuffe
     AttnTcArgs at = {attn, QSZ, D, 0, 0, NQ / NKV, 0, 8, 0, 0.08838834764831845f * 1.4426950408889634f, nullptr, status};
     at.tile_seq = tile_seq; at.tile_q0 = tile_q0; at.seq_len = seq_len; at.seq_row0 = seq_row0;
     at.seq_planes = model->num_layers * NKV;
+    at.qkv = qkv; at.k_cache = (const bf16*)bb->k_cache; at.v_cache = (const bf16*)bb->v_cache; at.plane_elems = (size_t)model->max_seq_len * D;
     launch_pdl(k_pf_embed, dim3(T), dim3(128), 0, stream, ids, (const bf16*)model->embed, h, model->vocab_size, status,
                (const bf16*)nullptr, 0, 0);
     Heads heads = {};
@@ -1149,12 +931,12 @@ static int decode_batch_impl(const MqModel* model, const MqBatchBuffers* bb, con
                            bb->attn_parts_bytes >= (size_t)B * NKV * BD_MAX_PARTS * 2 * BD_PART * sizeof(float);
     const BdShape shape = bd_shape(B * NKV, sm_count[dev_now], can_split);
     // up to 64 rows: the cluster chain (sk_chain.cuh), its row sums in the caller's scratch; above, tile GEMMs
-    const bool skinny = B <= 64 && bb->partials != nullptr && bb->partials_bytes >= (size_t)B * SK_SSQ * sizeof(float);
+    const bool skinny = B <= SK_MAX_ROWS && bb->partials != nullptr && bb->partials_bytes >= (size_t)B * SK_SSQ * sizeof(float);
     if (skinny) {
         SkArgs a = sk_args(model, B, h, bb->partials, (bf16*)bb->k_cache, (bf16*)bb->v_cache, status);
         a.pos_rows = bb->positions;
         a.seq_stride = seq_stride;
-        launch_pdl(k_sk_embed, dim3(B), dim3(128), 0, stream, in_tokens, (const bf16*)model->embed, h, a.ssq, model->vocab_size, status, (const bf16*)nullptr, 0, 0);
+        launch_pdl(k_sk_embed, dim3(B), dim3(128), 0, stream, in_tokens, (const bf16*)model->embed, h, a.ssq, model->vocab_size, status);
         for (int l = 0; l < model->num_layers; ++l) {
             rc = sk_qkv(model, l, a, qkv, stream);
             if (rc) return rc;

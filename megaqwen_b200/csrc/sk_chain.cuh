@@ -1,4 +1,4 @@
-// The linears of one layer for at most 128 rows (a decode step of a batch, a short prompt), each with the
+// The linears of one layer for at most 64 rows, a decode step of a batch, each with the
 // work around it: q|k|v with the norm before and QK-norm + RoPE + cache write behind, O and down with the
 // residual add, gate|up with the norm before and SwiGLU behind.
 //
@@ -8,10 +8,9 @@
 // the activation its N) and K is split over the CTAs of a CLUSTER, so that a linear spreads over 64 to 144 SMs with all
 // of a CTA's weights requested before the wait; the split's partial sums meet in distributed shared memory: rank r
 // of the cluster gets the rows [r TPC, (r + 1) TPC) of all partial tiles, adds them in rank order and
-// finishes those rows.  One layer used to be eight kernels with fp32 planes in global memory between them, a short
-// prompt took the 128-row tiles: step of batch 8 / 32 / 64 at contexts 400 / 384 / 1024 893 / 1107 / 2283 -> 747 / 967 / 2079 us;
-// prompt of 2 / 23 / 64 / 77 / 128 rows 1734 / 1812 / 1886 / 1897 / 1988 -> 750 / 764 / 974 / 1353 / 1540 us (weights alone: 184).
-// Where the two meet beyond 128 rows has not been looked for: the operands of one CTA fill its shared memory there.
+// finishes those rows.  One layer used to be eight kernels with fp32 planes in global memory between them: step of
+// batch 8 / 32 / 64 at contexts 400 / 384 / 1024 893 / 1107 / 2283 -> 747 / 967 / 2079 us.  The planes and the order in which they are
+// added are those of the eight kernels.  Prompts of as many rows do not come here: their sums over K are not split.
 //
 // RMSNorm: the kernel that finishes a row of the residual stream leaves the row's sum of squares of its 128 columns
 // in ssq[row][8]; the next linear adds the eight, normalises its K slice of the rows itself and writes it
@@ -23,26 +22,26 @@
 namespace mq {
 
 enum { SK_QKV = 0, SK_O = 1, SK_GU = 2, SK_DOWN = 3 };
-constexpr int SK_THREADS = 256, SK_BK = 64, SK_SSQ = H / 128, SK_MAX_ROWS = 128;
+constexpr int SK_THREADS = 256, SK_BK = 64, SK_SSQ = H / 128, SK_MAX_ROWS = 64;
 
 // Cluster sizes: 32 tiles x 4 = 128, 8 x 8 = 64 and 48 x 4 = 192 CTAs.  With one CTA to an SM the device holds 45 clusters of
-// three, 33 of four, 15 of eight; gate|up therefore keeps to 110 KB up to 64 rows, so that 71 clusters of four find room and its 48
+// three, 33 of four, 15 of eight; gate|up therefore keeps to 110 KB, so that 71 clusters of four find room and its 48
 // run in one round (one CTA an SM and three slices of K: two rounds, 12.0 against 4.9 us at 32 rows).
 template <int MPAD, int MODE>
 struct SkCfg {
     static constexpr int K = MODE == SK_O ? QSZ : MODE == SK_DOWN ? I : H;
-        static constexpr int KS = MODE == SK_QKV || MODE == SK_GU ? 4 : 8;
+    static constexpr int KS = MODE == SK_QKV || MODE == SK_GU ? 4 : 8;
     static constexpr int NKB = (K / SK_BK + KS - 1) / KS;                // k-blocks of one CTA, at most
     static constexpr int W_BYTES = 128 * SK_BK * 2, X_BYTES = MPAD * SK_BK * 2;
     static constexpr int TPC = (MPAD + KS - 1) / KS;                     // rows that one CTA of the cluster finishes
     static constexpr int RED_BYTES = KS * TPC * 128 * 4;
-    static constexpr bool ALIAS = NKB * (W_BYTES + X_BYTES) + RED_BYTES > (MODE == SK_GU && MPAD <= 64 ? 110 : 220) * 1024;   // the sums take the operands' place, behind one more barrier
+    static constexpr bool ALIAS = NKB * (W_BYTES + X_BYTES) + RED_BYTES > (MODE == SK_GU ? 110 : 220) * 1024;   // the sums take the operands' place, behind one more barrier
     static constexpr int RED_OFF = ALIAS ? 0 : NKB * (W_BYTES + X_BYTES);
     static constexpr int BAR_OFF = ALIAS ? NKB * (W_BYTES + X_BYTES) : RED_OFF + RED_BYTES;
     static constexpr size_t SMEM = (size_t)BAR_OFF + MPAD * 4 + 128 + 1024;
     static constexpr int TILES = MODE == SK_QKV ? QKV / 128 : MODE == SK_GU ? 2 * I / 128 : H / 128;
     static_assert((MODE != SK_QKV && MODE != SK_GU) || K == KS * 4 * SK_BK, "a K slice that is normed is 256 columns, eight a lane");
-    static_assert(MPAD % 16 == 0 && MPAD <= 128 && (!ALIAS || RED_BYTES <= NKB * (W_BYTES + X_BYTES)) && SMEM <= 232448, "one CTA's shared memory");
+    static_assert(MPAD % 16 == 0 && MPAD <= SK_MAX_ROWS && (!ALIAS || RED_BYTES <= NKB * (W_BYTES + X_BYTES)) && SMEM <= 232448, "one CTA's shared memory");
 };
 
 struct SkArgs {
@@ -51,11 +50,10 @@ struct SkArgs {
     float* ssq;                    // [M, 8] sums of squares of h by 128 columns: read (QKV, GU), written (O, DOWN)
     const bf16* gain;              // norm weight (QKV, GU)
     bf16* out;                     // QKV: [M, 4096], of which the rotated query heads are written; GU: [M, 3072]
-    // QKV: row s is position pos0 + s of one sequence or, with pos_rows, position pos_rows[s] of sequence s, whose caches begin
-    // s * seq_stride elements in
+    // QKV: row s is position pos_rows[s] of sequence s, whose caches begin s * seq_stride elements in
     const bf16 *q_norm, *k_norm, *cos, *sin;
     bf16 *k_cache, *v_cache;
-    int layer, pos0, max_seq;
+    int layer, max_seq;
     const int* pos_rows;
     size_t seq_stride;
     unsigned int* status;
@@ -181,7 +179,7 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
 #pragma unroll
         for (int i = 0; i < TW; ++i) {
             const int n = rank * TPC + warp + i * 8;
-            if (warp + i * 8 < TPC && n < a.M) pos[i] = a.pos_rows ? min(max(ld_cg_i32(a.pos_rows + n), 0), a.max_seq - 1) : a.pos0 + n;
+            if (warp + i * 8 < TPC && n < a.M) pos[i] = min(max(ld_cg_i32(a.pos_rows + n), 0), a.max_seq - 1);
         }
     }
     if (NORM) {
@@ -307,7 +305,7 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
                 uint32_t lo = pack_bf16x2(xl[0], xl[1]), hi = pack_bf16x2(xh[0], xh[1]);
                 if (!is_v) head_norm_rope(xl, xh, wl, wh, cl[i], ch[i], sl[i], sh[i], lo, hi);
                 const int head = is_q ? tile : is_v ? tile - (QSZ + KVSZ) / 128 : tile - QSZ / 128;
-                const size_t seq = a.pos_rows ? (size_t)n * a.seq_stride : 0;
+                const size_t seq = (size_t)n * a.seq_stride;
                 bf16* dst = is_q ? a.out + (size_t)n * QKV + tile * 128
                                  : (is_v ? a.v_cache : a.k_cache) + seq + ((size_t)(a.layer * NKV + head) * a.max_seq + pos[i]) * D;
                 *reinterpret_cast<uint32_t*>(dst + 2 * lane) = lo;
@@ -319,24 +317,18 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
     if (warp == 1) tmem_dealloc(tmem, TM_COLS);
 }
 
-// h[s,:] = embed[ids[s],:] (or the audio embedding of that row) and the row's sums of squares
+// h[s,:] = embed[ids[s],:] and the row's sums of squares
 __global__ void __launch_bounds__(128) k_sk_embed(const int* __restrict__ ids, const bf16* __restrict__ embed, bf16* __restrict__ h, float* __restrict__ ssq,
-                                                  int vocab, unsigned int* status, const bf16* __restrict__ audio, int audio_start, int audio_len) {
+                                                  int vocab, unsigned int* status) {
     pdl_wait();
     pdl_trigger();   // only now: the kernels behind may read cache rows of earlier steps ahead of their own waits
     const int s = blockIdx.x, tid = threadIdx.x;
-    const bf16* src;
-    if (audio != nullptr && s >= audio_start && s < audio_start + audio_len) {
-        src = audio + (size_t)(s - audio_start) * H;
-    } else {
-        int tok = ids[s];
-        if (tok < 0 || tok >= vocab) {
-            if (tid == 0) atomicOr(status, MQ_STATUS_BAD_TOKEN);
-            tok = min(max(tok, 0), vocab - 1);
-        }
-        src = embed + (size_t)tok * H;
+    int tok = ids[s];
+    if (tok < 0 || tok >= vocab) {
+        if (tid == 0) atomicOr(status, MQ_STATUS_BAD_TOKEN);
+        tok = min(max(tok, 0), vocab - 1);
     }
-    const uint4 u = __ldg(reinterpret_cast<const uint4*>(src) + tid);
+    const uint4 u = __ldg(reinterpret_cast<const uint4*>(embed + (size_t)tok * H) + tid);
     reinterpret_cast<uint4*>(h + (size_t)s * H)[tid] = u;
     const uint32_t x[4] = {u.x, u.y, u.z, u.w};
     float ss = 0.f;
@@ -381,7 +373,7 @@ static int launch_sk(const CUtensorMap& m0, const CUtensorMap& m1, const CUtenso
 template <int MODE>
 static int sk_linear(const MqLayerWeights& w, const bf16* x, SkArgs a, cudaStream_t stream) {
     CUtensorMap m0, m1, m2, mx;
-    const int mpad = a.M <= 16 ? 16 : a.M <= 32 ? 32 : a.M <= 64 ? 64 : 128;
+    const int mpad = a.M <= 16 ? 16 : a.M <= 32 ? 32 : 64;
     constexpr int K = SkCfg<16, MODE>::K;
     int rc;
     if (MODE == SK_QKV) {
@@ -402,8 +394,7 @@ static int sk_linear(const MqLayerWeights& w, const bf16* x, SkArgs a, cudaStrea
     switch (mpad) {
     case 16: return launch_sk<16, MODE>(m0, m1, m2, mx, a, stream);
     case 32: return launch_sk<32, MODE>(m0, m1, m2, mx, a, stream);
-    case 64: return launch_sk<64, MODE>(m0, m1, m2, mx, a, stream);
-    default: return launch_sk<128, MODE>(m0, m1, m2, mx, a, stream);
+    default: return launch_sk<64, MODE>(m0, m1, m2, mx, a, stream);
     }
 }
 

@@ -1,6 +1,7 @@
 // Causal attention on tcgen05 for a whole prompt, a portion of one, or several prompts packed row after row.
 #pragma once
 
+#include "mma_attention.cuh"
 #include "tc_gemm.cuh"
 
 namespace mq {
@@ -53,8 +54,12 @@ struct AttnTcArgs {
     // PACKED: prompts of several sequences row after row, positions from 0.  Query tile blockIdx.y begins at row tile_q0[y] of sequence
     // tile_seq[y]; sequence s has seq_len[s] rows from packed row seq_row0[s] on and its planes of the K and V maps, which are
     // max_seq rows long, from s * seq_planes on.
+    // A sequence below TA_BQ rows takes the mma.sync tiles that it takes alone, from the arrays behind the maps: the same bits
+    // whether it is packed or not.
     const int *tile_seq = nullptr, *tile_q0 = nullptr, *seq_len = nullptr, *seq_row0 = nullptr;
     int seq_planes = 0;
+    const bf16 *qkv = nullptr, *k_cache = nullptr, *v_cache = nullptr;
+    size_t plane_elems = 0;
 };
 
 // Maps: tmQ [head][token][d], tmK and tmV [plane][key][d] (the keys end at the last one of the prompt); with RP > 0
@@ -80,6 +85,18 @@ k_attention_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     }
     extern __shared__ uint8_t ta_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ta_raw) + 1023) & ~(uintptr_t)1023);
+    if constexpr (PACKED) {
+        if (S < TA_BQ) {                         // the same for the whole CTA
+            static_assert(FA_SMEM + 1024 <= Cfg::SMEM && FA_THREADS <= TA_THREADS && 2 * FA_BQ == TA_BQ, "a tile is up to two of the other kernel");
+            if (threadIdx.x >= FA_THREADS) return;
+            const size_t plane = (size_t)(plane0 + (int)blockIdx.x / a.kv_group) * a.plane_elems;
+            for (int q = 0; q < S; q += FA_BQ) {
+                __syncthreads();                 // the tile before this one has been merged
+                fa_tile(smem, a.qkv + (size_t)row0 * QKV, a.k_cache + plane, a.v_cache + plane, a.out + (size_t)row0 * a.ld_out, S, 0, q, (int)blockIdx.x);
+            }
+            return;
+        }
+    }
     uint8_t* sQ = smem;
     uint8_t* sK = sQ + Cfg::Q_BYTES;             // [2]
     uint8_t* sV = sK + 2 * Cfg::Q_BYTES;         // [2]
