@@ -16,127 +16,109 @@ int sm_count() {
 }
 
 // ---------------------------------------------------------------- 32-bit
-// Bound by the FMA pipes from some thirty rows on (128 a clock and SM) and by the weights' bytes below.  A CTA makes
-// 4 RI x 64 outputs; its four warps deal the K steps of 16 among themselves (step w, w + 4, ..), each with a
-// three-stage ring of its own that it fills by cp.async two steps ahead, so no block barrier stands in the loop and a
-// prompt of a few dozen rows still spreads over every SM: tile and split are small because M is (a 64 x 64 tile of one
-// 16-step buffer took 547 us a product at 150 rows, all of it latency).  A thread holds RI x 8 outputs at a distance
-// of 4 rows and 8 columns, so that eight lanes read eight rows of the padded tile in one wavefront without a bank
-// conflict: 8 + RI loads of 16 bytes for 32 RI FMAs.  The warps' sums meet in shared memory in warp order, and the
-// sink sees 32 columns of a row, as from the tensor-core kernel.  Rows per tile (pick_rows): 8 or 16 where fewer than
-// half of 32 would be used, as the padding is multiplied too.
-// 150 rows, a 28-layer model of width 1024: all products of the prompt 33 -> 6 ms (23 TFLOP/s).
-constexpr int FN = 64, FK = 16, FLD = FK + 4, F_STAGES = 3, F_WARPS = 4;
-// two 32-bit FMAs, each rounded once: half the instructions (6144 x 1024 by 150 rows 72.6 -> 65.1 us), two chains of half the length
-__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
-template <int RI>
-constexpr size_t F32_SMEM = (size_t)F_WARPS * F_STAGES * (4 * RI + FN) * FLD * 4;
-template <int RI, bool PLANES>
-__global__ void __launch_bounds__(F_WARPS * 32) k_gemm_f32(const float* __restrict__ A, int lda, const float* __restrict__ W, int M, int N, int K,
-                                                           SegmentSink<float> sink, float* __restrict__ plane, int ldp) {
-    constexpr int FM = 4 * RI, STAGE = (FM + FN) * FLD, CLD = FN + 4;
-    static_assert((size_t)F_WARPS * FM * CLD * 4 <= F32_SMEM<RI>, "the warps' sums take the place of the rings");
+// Every output is one chain of FMAs over k, first to last, whatever the tile: K is split neither over CTAs nor over warps nor over
+// even and odd k.  (The 32-bit mode is what other implementations are compared with, and where a head's output nearly cancels
+// before its norm the order of a sum is what one sees: split sums took the logits of some prompts 7e-5 from where they were.)
+// Bound by the FMA pipes from some hundred rows on (128 a clock and SM) and below by the weights' bytes that few CTAs have in flight.
+// A CTA of four warps, two by two, makes 8 TI x 16 TJ outputs; a thread TI x TJ of them at a distance of 4 rows and 8 columns, so that
+// a warp's 16-byte loads of four k take one wavefront each: TI + TJ loads for 4 TI TJ FMAs.  Steps of FK k by cp.async into a ring
+// as deep as the tile is small, one block barrier each; the finished tile goes through shared memory so that the sink sees 32
+// columns of a row.  Prompt of 150 rows, 28 layers of width 1024: 27.9 -> 11.5 ms (64 x 64 tiles of one 16-step buffer before).
+constexpr int F_THREADS = 128;
+template <int TI_, int TJ_, int FK_, int STAGES_>
+struct F32Tile {
+    static constexpr int TI = TI_, TJ = TJ_, FK = FK_, STAGES = STAGES_;
+    static constexpr int M = 8 * TI, N = 16 * TJ, LD = FK + 4, STAGE = (M + N) * LD, CLD = N + 4, PASS = F_THREADS / (FK / 4);   // rows copied side by side
+    static constexpr size_t SMEM = (size_t)STAGES * STAGE * 4;
+    static_assert(N % 32 == 0 && N % PASS == 0 && M % PASS == 0 && FK % 16 == 0 && M * (N / 32) <= F_THREADS && M * CLD <= STAGES * STAGE,
+                  "a thread takes 32 columns of a row; the finished tile takes the place of the ring");
+};
+template <class Tile, bool PLANES>
+__global__ void __launch_bounds__(F_THREADS) k_gemm_f32(const float* __restrict__ A, int lda, const float* __restrict__ W, int M, int N, int K,
+                                                        SegmentSink<float> sink, float* __restrict__ plane, int ldp) {
+    constexpr int TI = Tile::TI, TJ = Tile::TJ, FK = Tile::FK, STAGES = Tile::STAGES, LD = Tile::LD;
     extern __shared__ __align__(16) float f32_ring[];
     pdl_trigger();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ty = lane >> 3, tx = lane & 7;
-    const int m0 = blockIdx.y * FM, n0 = blockIdx.x * FN;
-    const int steps = K / FK;                   // K is a multiple of 16
-    const int first = (int)((long long)blockIdx.z * steps / gridDim.z) + warp, end = (int)((long long)(blockIdx.z + 1) * steps / gridDim.z);
-    float* ring = f32_ring + warp * F_STAGES * STAGE;
-    const int lr = lane >> 2, lk = (lane & 3) * 4;                // a lane copies 16 bytes of every eighth row
-    auto load_w = [&](int s, int stage) {
-        float* dst = ring + stage * STAGE + (FM + lr) * FLD + lk;
-        const float* src = W + (size_t)(n0 + lr) * K + s * FK + lk;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int m0 = blockIdx.y * Tile::M, n0 = blockIdx.x * Tile::N;
+    const int row = (warp & 1) * 4 * TI + (lane >> 3), col = (warp >> 1) * 8 * TJ + (lane & 7);       // of this thread's first output
+    const int steps = (K + FK - 1) / FK;        // K is a multiple of 16: the last step may be part of one
+    const int lr = tid / (FK / 4), lk = tid % (FK / 4) * 4;
+    auto load_w = [&](int s) {
+        float* dst = f32_ring + (s % STAGES) * Tile::STAGE + (Tile::M + lr) * LD + lk;
+        const int k = s * FK + lk;
 #pragma unroll
-        for (int i = 0; i < FN / 8; ++i) {
-            const bool ok = n0 + lr + 8 * i < N;
-            cp_async16_zfill(dst + 8 * i * FLD, ok ? src + (size_t)8 * i * K : W, ok);
+        for (int i = 0; i < Tile::N; i += Tile::PASS) {
+            const bool ok = k < K && n0 + lr + i < N;
+            cp_async16_zfill(dst + i * LD, ok ? W + (size_t)(n0 + lr + i) * K + k : W, ok);
         }
     };
-    auto load_a = [&](int s, int stage) {
-        float* dst = ring + stage * STAGE + lr * FLD + lk;
-        const float* src = A + (size_t)(m0 + lr) * lda + s * FK + lk;
+    auto load_a = [&](int s) {
+        float* dst = f32_ring + (s % STAGES) * Tile::STAGE + lr * LD + lk;
+        const int k = s * FK + lk;
 #pragma unroll
-        for (int i = 0; i < FM / 8; ++i) {
-            const bool ok = m0 + lr + 8 * i < M;
-            cp_async16_zfill(dst + 8 * i * FLD, ok ? src + (size_t)8 * i * lda : A, ok);
+        for (int i = 0; i < Tile::M; i += Tile::PASS) {
+            const bool ok = k < K && m0 + lr + i < M;
+            cp_async16_zfill(dst + i * LD, ok ? A + (size_t)(m0 + lr + i) * lda + k : A, ok);
         }
     };
     // the weights do not hang on the kernel before this one
 #pragma unroll
-    for (int p = 0; p < F_STAGES - 1; ++p)
-        if (first + p * F_WARPS < end) load_w(first + p * F_WARPS, p);
+    for (int s = 0; s < STAGES - 1; ++s)
+        if (s < steps) load_w(s);
     pdl_wait();
 #pragma unroll
-    for (int p = 0; p < F_STAGES - 1; ++p) {
-        if (first + p * F_WARPS < end) load_a(first + p * F_WARPS, p);
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s < steps) load_a(s);
         cp_async_commit();
     }
-    uint64_t acc[RI][8] = {};                   // sums over the even and the odd k
-    int stage = 0;
-    for (int s = first; s < end; s += F_WARPS) {
-        cp_async_wait<F_STAGES - 2>();
-        __syncwarp();
-        {
-            const int sn = s + (F_STAGES - 1) * F_WARPS, to = stage == 0 ? F_STAGES - 1 : stage - 1;
-            if (sn < end) { load_w(sn, to); load_a(sn, to); }
-            cp_async_commit();
+    float acc[TI][TJ] = {};
+    for (int s = 0; s < steps; ++s) {
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();                        // step s has landed, for everybody, and the stage of step s - 1 has been read
+        if (s + STAGES - 1 < steps) { load_w(s + STAGES - 1); load_a(s + STAGES - 1); }
+        cp_async_commit();
+        const float* sa = f32_ring + (s % STAGES) * Tile::STAGE + row * LD;
+        const float* sb = f32_ring + (s % STAGES) * Tile::STAGE + (Tile::M + col) * LD;
+#pragma unroll
+        for (int k0 = 0; k0 < FK; k0 += 16) {
+            if (k0 > 0 && s * FK + k0 >= K) break;
+#pragma unroll
+            for (int k = k0; k < k0 + 16; k += 4) {
+                float4 av[TI], bv[TJ];
+#pragma unroll
+                for (int i = 0; i < TI; ++i) av[i] = load4(sa + 4 * i * LD + k);
+#pragma unroll
+                for (int j = 0; j < TJ; ++j) bv[j] = load4(sb + 8 * j * LD + k);
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+#pragma unroll
+                    for (int i = 0; i < TI; ++i)
+#pragma unroll
+                        for (int j = 0; j < TJ; ++j) acc[i][j] = fmaf((&av[i].x)[e], (&bv[j].x)[e], acc[i][j]);
+            }
         }
-        const float* sa = ring + stage * STAGE + ty * FLD;
-        const float* sb = ring + stage * STAGE + (FM + tx) * FLD;
-#pragma unroll
-        for (int k = 0; k < FK; k += 4) {
-            ulonglong2 av[RI], bv[8];
-#pragma unroll
-            for (int i = 0; i < RI; ++i) av[i] = *reinterpret_cast<const ulonglong2*>(sa + 4 * i * FLD + k);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) bv[j] = *reinterpret_cast<const ulonglong2*>(sb + 8 * j * FLD + k);
-#pragma unroll
-            for (int i = 0; i < RI; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    fma2(acc[i][j], av[i].x, bv[j].x);
-                    fma2(acc[i][j], av[i].y, bv[j].y);
-                }
-        }
-        __syncwarp();                           // the next iteration's copies overwrite what has just been read
-        stage = stage == F_STAGES - 1 ? 0 : stage + 1;
     }
     cp_async_wait_all();
     __syncthreads();
-    float* sums = f32_ring + warp * FM * CLD;
 #pragma unroll
-    for (int i = 0; i < RI; ++i)
+    for (int i = 0; i < TI; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            float2 t;
-            memcpy(&t, &acc[i][j], 8);
-            sums[(ty + 4 * i) * CLD + tx + 8 * j] = t.x + t.y;
-        }
+        for (int j = 0; j < TJ; ++j) f32_ring[(row + 4 * i) * Tile::CLD + col + 8 * j] = acc[i][j];
     __syncthreads();
-    if (tid < 2 * FM) {
-        const int r = tid >> 1, c = (tid & 1) * 32;
+    constexpr int PIECES = Tile::N / 32;
+    if (tid < Tile::M * PIECES) {
+        const int r = tid / PIECES, c = tid % PIECES * 32;
         if (m0 + r >= M || n0 + c >= N) return;
-        float v[32];
-        const float* p = f32_ring + r * CLD + c;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            float4 t = load4(p + 4 * q);
-#pragma unroll
-            for (int w = 1; w < F_WARPS; ++w) {
-                const float4 u = load4(p + w * FM * CLD + 4 * q);
-                t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
-            }
-            v[4 * q] = t.x; v[4 * q + 1] = t.y; v[4 * q + 2] = t.z; v[4 * q + 3] = t.w;
-        }
+        const float* p = f32_ring + r * Tile::CLD + c;
         if (PLANES) {                            // the plane is at least as wide as the tiles
-            float* out = plane + ((size_t)blockIdx.z * M + m0 + r) * ldp + n0 + c;
+            float* out = plane + (size_t)(m0 + r) * ldp + n0 + c;
 #pragma unroll
-            for (int q = 0; q < 8; ++q) store4(out + 4 * q, make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+            for (int q = 0; q < 8; ++q) store4(out + 4 * q, load4(p + 4 * q));
         } else {
             uint32_t u[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) u[j] = __float_as_uint(v[j]);
+            for (int j = 0; j < 32; ++j) u[j] = __float_as_uint(p[j]);
             sink(m0 + r, n0 + c, u);
         }
     }
@@ -171,43 +153,30 @@ static TileShape pick_tile(int M, int N, int kblocks, int max_split, int* split)
     return best;
 }
 
-// rows of a 32-bit tile: 32, or 16 or 8 where that leaves a fifth less padding to multiply
-static int pick_rows(int M) {
-    if (M <= 8) return 8;
-    const int p32 = (M + 31) / 32 * 32, p16 = (M + 15) / 16 * 16;
-    return 5 * p16 <= 4 * p32 ? 16 : 32;
-}
-template <int RI, bool PLANES>
-static int go_f32(Stream& st, const float* A, int lda, const float* W, int M, int N, int K, int split, const SegmentSink<float>& sink, float* plane, int ldp) {
-    const int rc = allow_smem(k_gemm_f32<RI, PLANES>, F32_SMEM<RI>);
+template <class Tile, bool PLANES>
+static int go_f32(Stream& st, const float* A, int lda, const float* W, int M, int N, int K, const SegmentSink<float>& sink, float* plane, int ldp) {
+    const int rc = allow_smem(k_gemm_f32<Tile, PLANES>, Tile::SMEM);
     if (rc) return rc;
-    return launch(st, k_gemm_f32<RI, PLANES>, dim3((N + FN - 1) / FN, (M + 4 * RI - 1) / (4 * RI), split), dim3(F_WARPS * 32), F32_SMEM<RI>, A, lda, W, M, N,
-                  K, sink, plane, ldp);
+    return launch(st, k_gemm_f32<Tile, PLANES>, dim3((N + Tile::N - 1) / Tile::N, (M + Tile::M - 1) / Tile::M), dim3(F_THREADS), Tile::SMEM, A, lda, W, M, N, K,
+                  sink, plane, ldp);
 }
 template <bool PLANES>
-static int gemm_f32(Stream& st, const float* A, int lda, const float* W, int M, int N, int K, int split, const SegmentSink<float>& sink, float* plane, int ldp) {
-    switch (pick_rows(M)) {
-    case 8: return go_f32<2, PLANES>(st, A, lda, W, M, N, K, split, sink, plane, ldp);
-    case 16: return go_f32<4, PLANES>(st, A, lda, W, M, N, K, split, sink, plane, ldp);
-    default: return go_f32<8, PLANES>(st, A, lda, W, M, N, K, split, sink, plane, ldp);
-    }
+static int gemm_f32(Stream& st, const float* A, int lda, const float* W, int M, int N, int K, const SegmentSink<float>& sink, float* plane, int ldp) {
+    // The narrower a tile, the more CTAs stream the weights of a product with N = 1024, and the deeper the rings; the wider, the more often
+    // a load serves.  Prompt of 8 / 64 / 100 / 150 / 300 rows, 28 layers of width 1024, with the first of these everywhere: 4.0 / 8.8 / 13.8 / 19.5 / 36.0 ms,
+    // the second: 4.9 / 7.6 / 10.0 / 15.3 / 24.8, the third: 6.3 / 9.2 / 10.2 / 11.5 / 19.6; 4 x 4 outputs a thread: 8.1 / 11.2 / 13.3 / 15.3 / 21.6.
+    if (M <= 8) return go_f32<F32Tile<1, 2, 64, 8>, PLANES>(st, A, lda, W, M, N, K, sink, plane, ldp);
+    if (M <= 96) return go_f32<F32Tile<2, 2, 64, 6>, PLANES>(st, A, lda, W, M, N, K, sink, plane, ldp);
+    return go_f32<F32Tile<4, 2, 32, 6>, PLANES>(st, A, lda, W, M, N, K, sink, plane, ldp);
 }
 template <>
 int linear_segments<float>(Stream& st, const float* A, int lda, const float* W, int M, int N, int K, const Segments& g, unsigned int*) {
-    return gemm_f32<false>(st, A, lda, W, M, N, K, 1, SegmentSink<float>{g}, nullptr, 0);
+    return gemm_f32<false>(st, A, lda, W, M, N, K, SegmentSink<float>{g}, nullptr, 0);
 }
 template <>
 int linear_planes<float>(Stream& st, const float* A, int lda, const float* W, float* planes, int M, int N, int K, int ldp, int* nplanes, unsigned int*) {
-    // as many planes as shorten the longest SM's work: rounds of two CTAs an SM times the steps of a warp, and three to begin and end
-    const int tiles = ((N + FN - 1) / FN) * ((M + pick_rows(M) - 1) / pick_rows(M)), slots = 2 * sm_count();
-    int best = 1;
-    long long cost = -1;
-    for (int z = 1; z <= *nplanes; ++z) {
-        const long long c = (long long)((tiles * z + slots - 1) / slots) * ((K / FK + z * F_WARPS - 1) / (z * F_WARPS) + 3);
-        if (cost < 0 || c < cost) { cost = c; best = z; }
-    }
-    *nplanes = best;
-    return gemm_f32<true>(st, A, lda, W, M, N, K, best, SegmentSink<float>{}, planes, ldp);
+    *nplanes = 1;
+    return gemm_f32<true>(st, A, lda, W, M, N, K, SegmentSink<float>{}, planes, ldp);
 }
 
 template <>
