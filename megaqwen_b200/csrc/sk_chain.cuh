@@ -135,6 +135,7 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    cluster_arrive();          // the shared memory of a CTA may be accessed once it is known to run: waited for ahead of the first access
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
 
     if (tid == 0) {
@@ -251,6 +252,8 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
     __syncwarp();
     mbar_wait(accum, 0, a.status);
     tc_fence_after();
+    __syncwarp();
+    cluster_wait();            // every CTA of the cluster has started, microseconds ago
     if (Cfg::ALIAS) {          // every CTA of the cluster has read its operands: their place may be written
         cluster_arrive();
         cluster_wait();

@@ -1,0 +1,53 @@
+"""Device code, read on the host: no kernel touches another CTA's shared memory before a barrier over the whole cluster has
+said that all of its CTAs run."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "megaqwen_b200", "csrc")
+ACCESS = re.compile(r"\b(?:cluster_map|st_cluster_f32|ld_cluster|leader_addr)\(")
+BARRIER = re.compile(r"\b(?:cluster_wait|cluster_sync|cluster_sync_all)\(\);")
+
+
+def bodies(text):
+    """(name, body) of every function, comments taken out."""
+    text = re.sub(r"//[^\n]*", "", text)
+    for m in re.finditer(r"\b(\w+)\(([^;{}]*)\) \{\n", text):
+        if m.group(1) in ("if", "for", "while", "switch"):
+            continue
+        depth, at = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[at], 0)
+            at += 1
+        kernel = re.search(r"\b(k_\w+)\(", m.group(0))              # behind its launch bounds
+        yield kernel.group(1) if kernel else m.group(1), text[m.end():at - 1]
+
+
+def first_access_without_barrier(body):
+    """Whether an access stands before any barrier that every thread of every variant passes (one at the outermost level)."""
+    depth = 0
+    for token in re.finditer(r"[{}]|" + ACCESS.pattern + "|" + BARRIER.pattern, body):
+        t = token.group(0)
+        if t in "{}":
+            depth += 1 if t == "{" else -1
+        elif BARRIER.match(t):
+            if depth == 0:
+                return False
+        else:
+            return True
+    return False
+
+
+@pytest.mark.parametrize("name", sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))))
+def test_cluster_barrier_before_the_first_access(name):
+    text = open(os.path.join(CSRC, name)).read()
+    helpers = {"cluster_map", "st_cluster_f32", "ld_cluster", "leader_addr"}
+    bad = [f for f, body in bodies(text) if f not in helpers and first_access_without_barrier(body)]
+    assert not bad, bad
+
+
+def test_the_rule_sees_the_kernels():
+    seen = {f for n in ("sk_chain.cuh", "tc_gemm2.cuh", "hy_attention.cu") for f, body in bodies(open(os.path.join(CSRC, n)).read()) if ACCESS.search(body)}
+    assert {"k_sk", "k_gemm2", "merge_pieces"} <= seen
+    assert first_access_without_barrier("x(); if (a) { cluster_wait(); } st_cluster_f32(p, v);")
