@@ -328,6 +328,12 @@ int mq_launch_gemm_bf16(const void* A, int lda, const void* B, void* C, const vo
 int mq_debug_gemm_drop_load(const void* A, int lda, const void* B, void* C, int M, int N, int K, int ldc,
                             unsigned int* status, void* stream, int drop_kb);
 
+/* The same for the cluster chain of mq_launch_decode_batch: one linear of layer 0 on what bb's buffers hold
+ * (which: 0 q|k|v, 1 O, 2 gate|up, 3 down; the row sums of squares in bb->partials).  drop >= 0: block drop % 16 of
+ * CTA drop / 16 of every cluster is never requested; no CTA of a cluster with a missing sum stores anything.
+ * drop = -1: the linear as in a step.  No production path uses it. */
+int mq_debug_chain_drop_load(const MqModel* model, const MqBatchBuffers* bb, int which, int drop, void* stream);
+
 /* Standalone bf16 ops with the rounding points of the fused kernels.  They
  * replace the reference's csrc/kernels launchers (declared in
  * csrc/kernels/__init__.py:40-95): launch_rms_norm (rms_norm.cu:60-170),

@@ -100,6 +100,7 @@ SIGNATURES = {
                                       C.c_int, C.c_void_p, C.c_void_p]),
     "mq_debug_gemm_drop_load": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int,
                                           C.c_void_p, C.c_void_p, C.c_int]),
+    "mq_debug_chain_drop_load": (C.c_int, [C.POINTER(MqModel), C.POINTER(MqBatchBuffers), C.c_int, C.c_int, C.c_void_p]),
     "mq_launch_rms_norm": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_float, C.c_void_p]),
     "mq_launch_silu_mul": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_longlong, C.c_void_p]),
     "mq_launch_rope": (C.c_int, [C.c_void_p] * 6 + [C.c_int] * 4 + [C.c_void_p]),

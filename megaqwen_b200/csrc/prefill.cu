@@ -620,6 +620,26 @@ static int sk_rest(const MqModel* model, int l, SkArgs a, const bf16* attn, bf16
     return rc ? rc : sk_linear<SK_DOWN>(w, act, a, stream);
 }
 
+// Test hook: one linear of layer 0 of the chain on what bb's buffers hold (which: 0 q|k|v, 1 O, 2 gate|up, 3 down).  drop >= 0: block
+// drop % 16 of CTA drop / 16 of every cluster is never requested, so that one of its waits runs out.  Not used by any production path.
+extern "C" int mq_debug_chain_drop_load(const MqModel* model, const MqBatchBuffers* bb, int which, int drop, void* stream_v) {
+    if (!model || !bb || !bb->k_cache || !bb->v_cache || !bb->positions || !bb->status || which < SK_QKV || which > SK_DOWN || drop < -1) return MQ_ERR_BAD_ARG;
+    const MqPrefillBuffers* pb = &bb->act;
+    if (!pb->h || !pb->qkv || !pb->attn || !pb->act || !bb->partials || bb->partials_bytes < (size_t)bb->batch * SK_SSQ * sizeof(float)) return MQ_ERR_BAD_ARG;
+    if (bb->batch < 1 || bb->batch > SK_MAX_ROWS || bb->batch > pb->max_tokens) return MQ_ERR_BAD_ARG;
+    cudaStream_t stream = (cudaStream_t)stream_v;
+    SkArgs a = sk_args(model, bb->batch, (bf16*)pb->h, bb->partials, (bf16*)bb->k_cache, (bf16*)bb->v_cache, bb->status);
+    a.pos_rows = bb->positions;
+    a.seq_stride = (size_t)model->num_layers * NKV * model->max_seq_len * D;
+    a.drop = drop;
+    if (which == SK_QKV) return sk_qkv(model, 0, a, (bf16*)pb->qkv, stream);
+    const MqLayerWeights& w = model->layers[0];
+    a.gain = (const bf16*)w.post_attn_layernorm;
+    a.out = (bf16*)pb->act;
+    return which == SK_O ? sk_linear<SK_O>(w, (const bf16*)pb->attn, a, stream) : which == SK_GU ? sk_linear<SK_GU>(w, nullptr, a, stream)
+                                                                                 : sk_linear<SK_DOWN>(w, (const bf16*)pb->act, a, stream);
+}
+
 // The linears of many rows.  A GEMM on pairs of SMs (tc_gemm2.cuh) has two microseconds more to set up (a cluster, two CTAs' barriers)
 // and one tile's epilogue to show at the end, but hides the others and streams at 1.2 to 1.4 PFLOP/s: it is taken as soon as
 // k_gemm's tiles would need a second round.  us per linear, weights from HBM, k_gemm / pair:

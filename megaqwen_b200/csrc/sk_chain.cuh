@@ -57,6 +57,7 @@ struct SkArgs {
     const int* pos_rows;
     size_t seq_stride;
     unsigned int* status;
+    int drop = -1;                 // test hook: block drop % 16 of rank drop / 16 of every cluster is never requested
 };
 
 // products of two pairs of bf16, each rounded once
@@ -118,8 +119,9 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + Cfg::BAR_OFF);    // [NKB]
     uint64_t* accum = full + Cfg::NKB;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
+    volatile uint32_t* bad = tmem_slot + 1;                               // a bounded wait of some CTA of the cluster has run out: its sums are missing
     float* inv = reinterpret_cast<float*>(smem + Cfg::BAR_OFF + 128);     // [MPAD]
-    static_assert((Cfg::NKB + 1) * 8 + 4 <= 128, "barriers");
+    static_assert((Cfg::NKB + 1) * 8 + 8 <= 128 && Cfg::NKB <= 16, "barriers");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tile = blockIdx.x, rank = blockIdx.y;                       // the cluster runs along y
     const int kb0 = rank * KB / KS, nkb = (rank + 1) * KB / KS - kb0;
@@ -128,6 +130,7 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
         for (int i = 0; i < Cfg::NKB; ++i) mbar_init(&full[i], 1);
         mbar_init(accum, 1);
         mbar_fence_init();
+        *bad = 0u;
     }
     if (warp == 1) tmem_alloc(tmem_slot, TM_COLS);
     uint4 gv = make_uint4(0u, 0u, 0u, 0u);                                // norm weights of this lane's eight columns
@@ -141,6 +144,7 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
     if (tid == 0) {
         // the weights hang on nothing: all of them are requested before the wait
         for (int i = 0; i < nkb; ++i) {
+            if (rank * 16 + i == a.drop) continue;
             uint8_t* w = smem + i * Cfg::W_BYTES;
             mbar_expect_tx(&full[i], (uint32_t)(Cfg::W_BYTES + (NORM ? 0 : Cfg::X_BYTES)));
             const int x = (kb0 + i) * SK_BK;
@@ -164,7 +168,8 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
     }
     pdl_wait();
     if (!NORM && tid == 0)
-        for (int i = 0; i < nkb; ++i) tma_load_2d(xs + i * Cfg::X_BYTES, &tmX, (kb0 + i) * SK_BK, 0, &full[i]);
+        for (int i = 0; i < nkb; ++i)
+            if (rank * 16 + i != a.drop) tma_load_2d(xs + i * Cfg::X_BYTES, &tmX, (kb0 + i) * SK_BK, 0, &full[i]);
     // what the rows that this CTA finishes need besides the sums; a warp takes rows warp, warp + 8, .. of them
     constexpr int TW = (TPC + 7) / 8;
     uint2 hv[TW] = {};
@@ -238,10 +243,11 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
             sh[i] = *reinterpret_cast<const uint32_t*>(s + 64 + 2 * lane);
         }
     }
+    bool ok = true;            // after an expired wait nothing more is issued, and no CTA of the cluster stores a result
     if (tid == 32) {
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MPAD >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
         for (int i = 0; i < nkb; ++i) {
-            mbar_wait(&full[i], 0, a.status);
+            if (!mbar_wait(&full[i], 0, a.status)) { ok = false; break; }
             tc_fence_after();
             const uint64_t dw = smem_desc_sw128(smem + i * Cfg::W_BYTES), dx = smem_desc_sw128(xs + i * Cfg::X_BYTES);
 #pragma unroll
@@ -250,15 +256,17 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
         umma_commit(accum);
     }
     __syncwarp();
-    mbar_wait(accum, 0, a.status);
+    if (!mbar_wait(accum, 0, a.status)) ok = false;
     tc_fence_after();
     __syncwarp();
     cluster_wait();            // every CTA of the cluster has started, microseconds ago
+    if (!ok)
+        for (int r = 0; r < KS; ++r) st_cluster_f32(cluster_map(smem_u32(tmem_slot + 1), r), 1u);
     if (Cfg::ALIAS) {          // every CTA of the cluster has read its operands: their place may be written
         cluster_arrive();
         cluster_wait();
     }
-    {
+    if (__all_sync(0xffffffffu, ok)) {
         // warp w reads lanes 32 (w % 4) .. (weight rows) and half of the columns (activation rows)
         constexpr int HALF = MPAD / 2;
         const int quarter = warp & 3, c0 = (warp >> 2) * HALF;
@@ -274,12 +282,14 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
         }
         tc_fence_before();
     }
+    __syncwarp();
     cluster_arrive();
     cluster_wait();
+    const bool store = *bad == 0u;                                        // the same for the whole cluster
 #pragma unroll
     for (int i = 0; i < TW; ++i) {
         const int t = warp + i * 8, n = rank * TPC + t;
-        if (t >= TPC || n >= a.M) continue;
+        if (t >= TPC || n >= a.M || !store) continue;
         const float* p = red + t * 128;
         if (MODE == SK_O || MODE == SK_DOWN) {
             float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -317,6 +327,13 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
         }
     }
     __syncthreads();
+    if (!store) {              // copies and products that were issued end before their memory is given back
+        if (tid == 0)
+            for (int i = 0; i < nkb; ++i)
+                if (rank * 16 + i != a.drop) mbar_wait_drain(&full[i], 0);
+        if (tid == 32) mbar_wait_drain(accum, 0);
+        __syncthreads();
+    }
     if (warp == 1) tmem_dealloc(tmem, TM_COLS);
 }
 

@@ -14,7 +14,7 @@ def bodies(text):
     """(name, body) of every function, comments taken out."""
     text = re.sub(r"//[^\n]*", "", text)
     for m in re.finditer(r"\b(\w+)\(([^;{}]*)\) \{\n", text):
-        if m.group(1) in ("if", "for", "while", "switch"):
+        if text[text.rfind("\n", 0, m.start()) + 1].isspace():               # a statement inside a function
             continue
         depth, at = 1, m.end()
         while depth:
