@@ -328,6 +328,12 @@ int mq_launch_gemm_bf16(const void* A, int lda, const void* B, void* C, const vo
 int mq_debug_gemm_drop_load(const void* A, int lda, const void* B, void* C, int M, int N, int K, int ldc,
                             unsigned int* status, void* stream, int drop_kb);
 
+/* The same for the GEMM on pairs of SMs, C = A B^T + R with N a multiple of 256: a pair of SMs computes several 256 x 256 tiles one
+ * after the other (pair p the tiles p, p + pairs, ..); drop_kb counts the k-blocks of one pair over all of its tiles, and
+ * the tiles before the one that lacks a block are stored.  drop_kb = -1: nothing is left out. */
+int mq_debug_gemm_pair_drop_load(const void* A, int lda, const void* B, void* C, const void* R, int M, int N, int K, int ldc,
+                                 unsigned int* status, void* stream, int drop_kb);
+
 /* The same for the cluster chain of mq_launch_decode_batch: one linear of layer 0 on what bb's buffers hold
  * (which: 0 q|k|v, 1 O, 2 gate|up, 3 down; the row sums of squares in bb->partials).  drop >= 0: block drop % 16 of
  * CTA drop / 16 of every cluster is never requested; no CTA of a cluster with a missing sum stores anything.

@@ -100,6 +100,8 @@ SIGNATURES = {
                                       C.c_int, C.c_void_p, C.c_void_p]),
     "mq_debug_gemm_drop_load": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int,
                                           C.c_void_p, C.c_void_p, C.c_int]),
+    "mq_debug_gemm_pair_drop_load": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int,
+                                               C.c_int, C.c_void_p, C.c_void_p, C.c_int]),
     "mq_debug_chain_drop_load": (C.c_int, [C.POINTER(MqModel), C.POINTER(MqBatchBuffers), C.c_int, C.c_int, C.c_void_p]),
     "mq_launch_rms_norm": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_float, C.c_void_p]),
     "mq_launch_silu_mul": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_longlong, C.c_void_p]),

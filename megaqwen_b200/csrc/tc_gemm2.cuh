@@ -106,6 +106,7 @@ struct Gemm2Args {
     const bf16* R;
     unsigned int* status;
     int early_b;                   // B is written by nothing on the stream
+    int drop_kb;                   // test hook: the k-block, counted over a pair's tiles, that is never requested; -1 in every production launch
 };
 
 template <int BN, int EPI, class Sink = NoSink>
@@ -166,15 +167,16 @@ k_gemm2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtenso
         }
     };
 
+    int c = 0;                                // k-blocks requested so far, over all tiles (producer)
     if (warp == 0) {
         if (lane == 0) {
-            int c = 0;                        // k-blocks requested so far, over all tiles
             int npre = 0;
             if (a.early_b && first < tiles) { // the first tile's weights, ring permitting, before the preceding grid has finished
                 int tm, tn, z, kb0, nk;
                 place(first, tm, tn, z, kb0, nk);
                 npre = nk < ST ? nk : ST;
                 for (int i = 0; i < npre; ++i) {
+                    if (i == a.drop_kb) continue;
                     if (leader) mbar_expect_tx(&full[i], 2 * Cfg::STAGE_BYTES);
                     load_b(smem + (size_t)i * Cfg::STAGE_BYTES, leader_addr(&full[i]), tn, kb0 + i);
                 }
@@ -186,6 +188,7 @@ k_gemm2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtenso
                 for (int i = 0; i < nk; ++i, ++c) {
                     const int s = c % ST;
                     if (c >= ST && !mbar_wait(&empty[s], (uint32_t)(c / ST - 1) & 1u, a.status)) { *aborted = 1u; break; }
+                    if (c == a.drop_kb) continue;
                     uint8_t* st = smem + (size_t)s * Cfg::STAGE_BYTES;
                     const uint32_t bar = leader_addr(&full[s]);
                     if (c >= npre && leader) mbar_expect_tx(&full[s], 2 * Cfg::STAGE_BYTES);
@@ -193,15 +196,13 @@ k_gemm2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtenso
                     if (c >= npre) load_b(st, bar, tn, kb0 + i);
                 }
             }
-            if (*aborted && leader)           // copies that were requested still land: wait for the last of every stage, with a limit
-                for (int s = 0; s < ST && s < c; ++s) mbar_wait_drain(&full[s], (uint32_t)(((c - 1 - s) / ST)) & 1u);
         }
         __syncwarp();
     } else if (warp == 1) {
         if (leader && lane == 0) {
             // D = f32, A = B = bf16, both K-major, N >> 3, M = 256 >> 4
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
-            int c = 0, it = 0;
+            int it = 0;
             for (int t = first; t < tiles && !*aborted; t += step, ++it) {
                 int tm, tn, z, kb0, nk;
                 place(t, tm, tn, z, kb0, nk);
@@ -342,6 +343,16 @@ k_gemm2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtenso
         }
         tc_fence_before();
     }
+    __syncthreads();
+    // After an expired wait (which the other CTA of the pair then runs into as well): copies that were requested still land.  The leader
+    // waits for the last of every stage; the other CTA, whose copies report to the leader's barriers, for as long as the leader waits
+    // for one of them at most.
+    if (*aborted && tid == 0) {
+        if (leader)
+            for (int s = 0; s < ST && s < c; ++s) mbar_wait_drain(&full[s], (uint32_t)(((c - 1 - s) / ST)) & 1u);
+        else
+            mbar_wait_drain(drained, 0);      // nothing arrives there
+    }
     __syncwarp();
     cluster_sync_all();                       // both CTAs' copies, products and remote arrivals are done
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)Cfg::TMEM_COLS) : "memory");
@@ -351,7 +362,7 @@ k_gemm2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtenso
 // for planes at least as wide as the tiles.
 template <int BN, int EPI, class Sink = NoSink>
 static int launch_gemm2(const bf16* A, int lda, const bf16* B, const bf16* B2, bf16* C, const bf16* R, int M, int N, int K, int ldc, unsigned int* status,
-                        cudaStream_t stream, const bf16* B3 = nullptr, int rows0 = 0, int rows1 = 0, int ksplit = 1, bool early_b = true, Sink sink = Sink()) {
+                        cudaStream_t stream, const bf16* B3 = nullptr, int rows0 = 0, int rows1 = 0, int ksplit = 1, bool early_b = true, Sink sink = Sink(), int drop_kb = -1) {
     using Cfg = Gemm2Cfg<BN, EPI>;
     static int sms[64] = {0};
     int dev = 0;
@@ -384,7 +395,7 @@ static int launch_gemm2(const bf16* A, int lda, const bf16* B, const bf16* B2, b
         if (rc == MQ_OK) rc = get_map(B3, (uint64_t)(N - rows0 - rows1), (uint64_t)K, (uint64_t)K, BN / 2, &mb3);
     }
     if (rc != MQ_OK) return rc;
-    a.M = M; a.N = N; a.K = K; a.ldc = ldc; a.C = C; a.R = R; a.status = status; a.early_b = early_b ? 1 : 0;
+    a.M = M; a.N = N; a.K = K; a.ldc = ldc; a.C = C; a.R = R; a.status = status; a.early_b = early_b ? 1 : 0; a.drop_kb = drop_kb;
     a.tiles0 = concat ? rows0 / BN : (1 << 30);
     a.tiles1 = concat ? rows1 / BN : 0;
     const int tiles = a.tiles_m * a.tiles_n * ksplit, pairs = sms[dev] / 2;

@@ -46,3 +46,33 @@ def test_chain_of_a_batch(which, batch):
         assert all(torch.equal(t, s) for t, s in zip(state, start)), drop
         assert run(-1) == 0
         assert all(torch.equal(t, s) for t, s in zip(state, right)), drop
+
+
+@pytest.mark.parametrize("m,k,drop,whole", [(300, 1024, 0, 0), (300, 1024, 9, 0), (300, 128, 1, 0), (256 * 80, 128, 3, 74), (256 * 80, 1024, 31, 74)])
+def test_gemm_on_pairs(m, k, drop, whole):
+    """``whole``: 256-row tiles ahead of the first one that lacks a block, on 74 pairs of SMs (the last two cases drop a block of a pair's second tile)."""
+    lib = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    a, b, r = (torch.randn(s, generator=g, device="cuda", dtype=torch.bfloat16) for s in ((m, k), (256, k), (m, 256)))
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def run(drop_kb):
+        c = torch.full((m, 256), 7.0, dtype=torch.bfloat16, device="cuda")
+        status.zero_()
+        rc = lib.mq_debug_gemm_pair_drop_load(a.data_ptr(), k, b.data_ptr(), c.data_ptr(), r.data_ptr(), m, 256, k, 256, status.data_ptr(),
+                                              torch.cuda.current_stream().cuda_stream, drop_kb)
+        _lib.check(rc, "mq_debug_gemm_pair_drop_load")
+        torch.cuda.synchronize()
+        return c, int(status)
+
+    right, st = run(-1)
+    ref = (a.float() @ b.float().T).bfloat16().float() + r.float()
+    assert st == 0 and float((right.float() - ref).abs().max()) <= 2 ** -7 * float(ref.abs().max())
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        whole = 0 if whole == 0 else None
+    c, st = run(drop)
+    assert st == _lib.MQ_STATUS_WAIT_TIMEOUT
+    if whole is not None:
+        assert torch.equal(c[:256 * whole], right[:256 * whole]) and bool((c[256 * whole:] == 7.0).all())
+    again, st = run(-1)
+    assert st == 0 and torch.equal(again, right)
