@@ -67,7 +67,7 @@ __device__ __forceinline__ void fa_tile(uint8_t* fa_smem, const bf16* qkv, const
     for (int c = tid; c < FA_BQ * (D / 8); c += FA_THREADS) {
         const int r = c / (D / 8), cc = c % (D / 8);
         uint4 v = make_uint4(0, 0, 0, 0);
-        if (q0 + r < S) v = *reinterpret_cast<const uint4*>(qkv + (size_t)(q0 + r) * QKV + head * D + cc * 8);
+        if (q0 + r < S) v = ld_cg_u4(qkv + (size_t)(q0 + r) * QKV + head * D + cc * 8);
         *reinterpret_cast<uint4*>(sq + r * FA_LD + cc * 8) = v;
     }
     __syncthreads();

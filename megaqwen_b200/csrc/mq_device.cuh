@@ -54,7 +54,8 @@ __device__ __forceinline__ float warp_max(float v) {
 // ---------------------------------------------------------------- loads
 // Activations are rewritten by every kernel of the chain while kernels overlap
 // under programmatic dependent launch, so they are always read through L2
-// (ld.global.cg), never through a possibly stale L1 line.
+// (ld.global.cg), never through a possibly stale L1 line.  The same goes for tokens, positions and tables: a plain load of a
+// `const T* __restrict__` may even be moved ahead of the wait for the kernel that writes it, so only weights have that type.
 __device__ __forceinline__ uint4 ld_cg_u4(const void* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
 __device__ __forceinline__ uint2 ld_cg_u2(const void* p) { return __ldcg(reinterpret_cast<const uint2*>(p)); }
 __device__ __forceinline__ uint32_t ld_cg_u32(const void* p) { return __ldcg(reinterpret_cast<const uint32_t*>(p)); }

@@ -24,16 +24,16 @@
 namespace mq {
 
 // h = bf16(h + bf16(sum of the two fp32 planes of a K split));  x = rmsnorm(h) * w      one CTA per row (N = 1024), 4 columns per thread
-__global__ void __launch_bounds__(256) k_sk_resid_norm(const float* __restrict__ part, int M, bf16* __restrict__ h,
+__global__ void __launch_bounds__(256) k_sk_resid_norm(const float* part, int M, bf16* __restrict__ h,
                                                        const bf16* __restrict__ w, bf16* __restrict__ x) {
     pdl_trigger();   // the next grid may be scheduled already (it waits the same way)
     pdl_wait();      // launched with programmatic stream serialisation: the preceding grid has completed
     __shared__ float s_red[8];
     const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const size_t base = (size_t)row * H + 4 * tid, plane = (size_t)M * H;
-    const uint2 hu = *reinterpret_cast<const uint2*>(h + base);
+    const uint2 hu = ld_cg_u2(h + base);
     const uint2 wu = w ? *reinterpret_cast<const uint2*>(w + 4 * tid) : make_uint2(0u, 0u);   // requested with the planes, used after the row sum
-    const float4 p0 = *reinterpret_cast<const float4*>(part + base), p1 = *reinterpret_cast<const float4*>(part + plane + base);
+    const float4 p0 = __ldcg(reinterpret_cast<const float4*>(part + base)), p1 = __ldcg(reinterpret_cast<const float4*>(part + plane + base));
     const float4 acc = make_float4(p0.x + p1.x, p0.y + p1.y, p0.z + p1.z, p0.w + p1.w);
     float v[4] = {rbf(bf_lo(hu.x) + rbf(acc.x)), rbf(bf_hi(hu.x) + rbf(acc.y)), rbf(bf_lo(hu.y) + rbf(acc.z)), rbf(bf_hi(hu.y) + rbf(acc.w))};
     *reinterpret_cast<uint2*>(h + base) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(256) k_sk_resid_norm(const float* __restrict__
 // h[s,:] = embed[ids[s],:]      (reference: prefill_embed_kernel, fused_prefill_kernels.inl:3-20)
 // Rows audio_start .. audio_start + audio_len - 1 take externally computed embeddings instead
 // (reference: prefill_patch_audio_kernel, fused_prefill_kernels.inl:28-45, a separate launch there).
-__global__ void __launch_bounds__(128) k_pf_embed(const int* __restrict__ ids, const bf16* __restrict__ embed, bf16* __restrict__ h,
+__global__ void __launch_bounds__(128) k_pf_embed(const int* ids, const bf16* __restrict__ embed, bf16* __restrict__ h,
                                                   int vocab, unsigned int* status, const bf16* __restrict__ audio = nullptr,
                                                   int audio_start = 0, int audio_len = 0) {
     pdl_wait();      // launched with programmatic stream serialisation: the preceding grid has completed
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(128) k_pf_embed(const int* __restrict__ ids, c
             __ldg(reinterpret_cast<const uint4*>(audio + (size_t)(s - audio_start) * H) + threadIdx.x);
         return;
     }
-    int tok = ids[s];
+    int tok = ld_cg_i32(ids + s);
     if (tok < 0 || tok >= vocab) {
         if (threadIdx.x == 0) atomicOr(status, MQ_STATUS_BAD_TOKEN);
         tok = min(max(tok, 0), vocab - 1);
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(128) k_pf_embed(const int* __restrict__ ids, c
 
 // x[s,:] = bf16( w * bf16( h[s,:] * rsqrt(mean(h^2) + eps) ) )   one warp per row
 // (reference: prefill_rmsnorm_kernel, fused_prefill_kernels.inl:52-105)
-__global__ void __launch_bounds__(256) k_pf_rmsnorm(const bf16* __restrict__ h, const bf16* __restrict__ w, bf16* __restrict__ x, int rows) {
+__global__ void __launch_bounds__(256) k_pf_rmsnorm(const bf16* h, const bf16* __restrict__ w, bf16* __restrict__ x, int rows) {
     pdl_trigger();   // the next grid may be scheduled already (it waits the same way)
     pdl_wait();      // launched with programmatic stream serialisation: the preceding grid has completed
     const int lane = threadIdx.x & 31;
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(256) k_pf_rmsnorm(const bf16* __restrict__ h, 
     const bf16* src = h + (size_t)row * H;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const uint4 u = *reinterpret_cast<const uint4*>(src + j * 256 + lane * 8);
+        const uint4 u = ld_cg_u4(src + j * 256 + lane * 8);
         v[j * 8 + 0] = bf_lo(u.x); v[j * 8 + 1] = bf_hi(u.x); v[j * 8 + 2] = bf_lo(u.y); v[j * 8 + 3] = bf_hi(u.y);
         v[j * 8 + 4] = bf_lo(u.z); v[j * 8 + 5] = bf_hi(u.z); v[j * 8 + 6] = bf_lo(u.w); v[j * 8 + 7] = bf_hi(u.w);
     }
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(256) k_pf_rmsnorm(const bf16* __restrict__ h, 
 __global__ void __launch_bounds__(256) k_pf_qknorm_rope(bf16* __restrict__ qkv, const bf16* __restrict__ wq, const bf16* __restrict__ wk,
                                                         const bf16* __restrict__ cos, const bf16* __restrict__ sin, bf16* __restrict__ k_cache,
                                                         bf16* __restrict__ v_cache, int layer, int pos0, int max_seq,
-                                                        const int* __restrict__ pos_rows, size_t seq_stride, const int* __restrict__ row_seq) {
+                                                        const int* pos_rows, size_t seq_stride, const int* row_seq) {
     pdl_trigger();   // the next grid may be scheduled already (it waits the same way)
     pdl_wait();      // launched with programmatic stream serialisation: the preceding grid has completed
     // pos_rows == nullptr: one sequence, row s sits at position pos0 + s.
@@ -117,9 +117,9 @@ __global__ void __launch_bounds__(256) k_pf_qknorm_rope(bf16* __restrict__ qkv, 
     // then every gridDim.y * 8 further: one CTA per row with gridDim.y = 1, four with 4.
     const int lane = threadIdx.x & 31;
     const int s = blockIdx.x;
-    const int pos = pos_rows ? min(max(pos_rows[s], 0), max_seq - 1) : pos0 + s;
+    const int pos = pos_rows ? min(max(ld_cg_i32(pos_rows + s), 0), max_seq - 1) : pos0 + s;
     if (pos_rows) {
-        const size_t seq = row_seq ? (size_t)row_seq[s] : (size_t)s;
+        const size_t seq = row_seq ? (size_t)ld_cg_i32(row_seq + s) : (size_t)s;
         k_cache += seq * seq_stride;
         v_cache += seq * seq_stride;
     }
@@ -132,13 +132,13 @@ __global__ void __launch_bounds__(256) k_pf_qknorm_rope(bf16* __restrict__ qkv, 
         if (unit >= NQ + NKV) {   // V head: raw copy into the cache
             const int g = unit - NQ - NKV;
             *reinterpret_cast<uint2*>(v_cache + ((size_t)(layer * NKV + g) * max_seq + pos) * D + 4 * lane) =
-                *reinterpret_cast<const uint2*>(row + QSZ + KVSZ + g * D + 4 * lane);
+                ld_cg_u2(row + QSZ + KVSZ + g * D + 4 * lane);
             continue;
         }
         const bool is_q = unit < NQ;
         bf16* head = is_q ? row + unit * D : row + QSZ + (unit - NQ) * D;
         const bf16* wn = is_q ? wq : wk;
-        const uint32_t ulo = *reinterpret_cast<const uint32_t*>(head + 2 * lane), uhi = *reinterpret_cast<const uint32_t*>(head + 64 + 2 * lane);
+        const uint32_t ulo = ld_cg_u32(head + 2 * lane), uhi = ld_cg_u32(head + 64 + 2 * lane);
         const float xl[2] = {bf_lo(ulo), bf_hi(ulo)}, xh[2] = {bf_lo(uhi), bf_hi(uhi)};
         uint32_t plo, phi;
         head_norm_rope(xl, xh, *reinterpret_cast<const uint32_t*>(wn + 2 * lane), *reinterpret_cast<const uint32_t*>(wn + 64 + 2 * lane), cl, ch, sl, sh, plo, phi);
@@ -149,8 +149,7 @@ __global__ void __launch_bounds__(256) k_pf_qknorm_rope(bf16* __restrict__ qkv, 
 }
 
 // ---------------------------------------------------------------- causal GQA attention of a prompt below 128 rows
-__global__ void __launch_bounds__(FA_THREADS, 1) k_pf_attention(const bf16* __restrict__ qkv, const bf16* __restrict__ k_cache,
-                                                               const bf16* __restrict__ v_cache, bf16* __restrict__ out, int S, int pos0,
+__global__ void __launch_bounds__(FA_THREADS, 1) k_pf_attention(const bf16* qkv, const bf16* k_cache, const bf16* v_cache, bf16* out, int S, int pos0,
                                                                int layer, int max_seq) {
     pdl_trigger();   // the next grid may be scheduled already (it waits the same way)
     pdl_wait();      // launched with programmatic stream serialisation: the preceding grid has completed
@@ -165,20 +164,19 @@ __global__ void __launch_bounds__(FA_THREADS, 1) k_pf_attention(const bf16* __re
 // defined in decode.cu: final RMSNorm + LM head + arg-max on buf->hidden
 int launch_lmhead_only(const MqModel* model, const MqDecodeBuffers* buf, int* out_token, float* logits, cudaStream_t stream);
 
-__global__ void k_pf_copy_row(const bf16* __restrict__ src, bf16* __restrict__ dst) {
+__global__ void k_pf_copy_row(const bf16* src, bf16* __restrict__ dst) {
     pdl_trigger();   // the next grid may be scheduled already (it waits the same way)
     pdl_wait();      // launched with programmatic stream serialisation: the preceding grid has completed
-    reinterpret_cast<uint4*>(dst)[threadIdx.x] = reinterpret_cast<const uint4*>(src)[threadIdx.x];
+    reinterpret_cast<uint4*>(dst)[threadIdx.x] = ld_cg_u4(src + threadIdx.x * 8);
 }
 
 // dst[b] = src[last packed row of sequence b]
-__global__ void k_pf_gather_last(const bf16* __restrict__ src, const int* __restrict__ seq_row0, const int* __restrict__ seq_len,
-                                 bf16* __restrict__ dst) {
+__global__ void k_pf_gather_last(const bf16* src, const int* seq_row0, const int* seq_len, bf16* __restrict__ dst) {
     pdl_trigger();   // the next grid may be scheduled already (it waits the same way)
     pdl_wait();      // launched with programmatic stream serialisation: the preceding grid has completed
     const int b = blockIdx.x;
-    const size_t row = (size_t)seq_row0[b] + (size_t)seq_len[b] - 1;
-    reinterpret_cast<uint4*>(dst + (size_t)b * H)[threadIdx.x] = reinterpret_cast<const uint4*>(src + row * H)[threadIdx.x];
+    const size_t row = (size_t)ld_cg_i32(seq_row0 + b) + (size_t)ld_cg_i32(seq_len + b) - 1;
+    reinterpret_cast<uint4*>(dst + (size_t)b * H)[threadIdx.x] = ld_cg_u4(src + row * H + threadIdx.x * 8);
 }
 
 }  // namespace mq
@@ -261,10 +259,10 @@ __device__ __forceinline__ void bd_expand_tile_fp8(const uint8_t* raw, bf16* til
 // of a split item write their (m, l, acc) to `parts` and take a ticket, and the one that takes the last
 // merges them (no CTA waits for another).  tickets: one zero-initialised counter per item, reset by the merger.
 template <bool FP8, int WARPS>
-__device__ __forceinline__ void bd_attention_body(const bf16* __restrict__ qkv, const bf16* __restrict__ k_cache, const bf16* __restrict__ v_cache,
-                                                  bf16* __restrict__ out, const int* __restrict__ positions, int layer, int max_seq,
+__device__ __forceinline__ void bd_attention_body(const bf16* qkv, const bf16* k_cache, const bf16* v_cache,
+                                                  bf16* out, const int* positions, int layer, int max_seq,
                                                   size_t seq_stride, uint8_t* __restrict__ k8, uint8_t* __restrict__ v8,
-                                                  const float* __restrict__ k_scale, const float* __restrict__ v_scale, int scale_stride,
+                                                  const float* k_scale, const float* v_scale, int scale_stride,
                                                   float* __restrict__ parts, unsigned int* __restrict__ tickets, int n_full, int p_tail) {
     constexpr int BD_THREADS = WARPS * 32;
     const int cta = (int)blockIdx.x;
@@ -275,8 +273,8 @@ __device__ __forceinline__ void bd_attention_body(const bf16* __restrict__ qkv, 
     // the scales are set by the quantise kernel before the first step and constant afterwards
     float ks = 1.f, vs = 1.f;
     if constexpr (FP8) {
-        ks = kv_fp8_scale_guard(k_scale[(size_t)b * scale_stride + layer * NKV + g]);
-        vs = kv_fp8_scale_guard(v_scale[(size_t)b * scale_stride + layer * NKV + g]);
+        ks = kv_fp8_scale_guard(ld_cg_f32(k_scale + (size_t)b * scale_stride + layer * NKV + g));
+        vs = kv_fp8_scale_guard(ld_cg_f32(v_scale + (size_t)b * scale_stride + layer * NKV + g));
     }
     pdl_trigger();   // the next grid may be scheduled already (it waits the same way)
     extern __shared__ __align__(128) uint8_t bd_smem[];
@@ -284,7 +282,7 @@ __device__ __forceinline__ void bd_attention_body(const bf16* __restrict__ qkv, 
     bf16* qs = ring + (size_t)(BD_THREADS / 32) * BD_STAGES * BD_STAGE_ELEMS;         // [2][D]
     bf16* ps = qs + 2 * D;                                                            // [12 warps][2][16]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int pos = min(max(positions[b], 0), max_seq - 1);
+    const int pos = min(max(ld_cg_i32(positions + b), 0), max_seq - 1);
     const int len = pos + 1;
     const int ntiles_all = (len + 15) >> 4;
     // this CTA's share of the item's key tiles: [tile_lo, ntiles)
@@ -335,7 +333,7 @@ __device__ __forceinline__ void bd_attention_body(const bf16* __restrict__ qkv, 
     }
     if (tid >= 64 && tid < 96) {
         const int t8 = tid - 64;
-        uint4 q = ld_cg_u4(qkv + (size_t)b * QKV + 2 * g * D + t8 * 8);     // (a plain load of a restricted pointer may be moved ahead of the wait)
+        uint4 q = ld_cg_u4(qkv + (size_t)b * QKV + 2 * g * D + t8 * 8);
         if constexpr (FP8) {   // f16 tiles are multiplied with an f16 query
             q.x = pack_f16x2(bf_lo(q.x), bf_hi(q.x)); q.y = pack_f16x2(bf_lo(q.y), bf_hi(q.y));
             q.z = pack_f16x2(bf_lo(q.z), bf_hi(q.z)); q.w = pack_f16x2(bf_lo(q.w), bf_hi(q.w));
@@ -514,16 +512,16 @@ __device__ __forceinline__ void bd_attention_body(const bf16* __restrict__ qkv, 
 
 template <bool FP8, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 6 ? 2 : 1)
-k_bd_attention(const bf16* __restrict__ qkv, const bf16* __restrict__ k_cache, const bf16* __restrict__ v_cache, bf16* __restrict__ out,
-               const int* __restrict__ positions, int layer, int max_seq, size_t seq_stride, uint8_t* __restrict__ k8, uint8_t* __restrict__ v8,
-               const float* __restrict__ k_scale, const float* __restrict__ v_scale, int scale_stride, float* __restrict__ parts,
+k_bd_attention(const bf16* qkv, const bf16* k_cache, const bf16* v_cache, bf16* out,
+               const int* positions, int layer, int max_seq, size_t seq_stride, uint8_t* __restrict__ k8, uint8_t* __restrict__ v8,
+               const float* k_scale, const float* v_scale, int scale_stride, float* __restrict__ parts,
                unsigned int* __restrict__ tickets, int n_full, int p_tail) {
     bd_attention_body<FP8, WARPS>(qkv, k_cache, v_cache, out, positions, layer, max_seq, seq_stride, k8, v8, k_scale, v_scale, scale_stride, parts,
                                   tickets, n_full, p_tail);
 }
 
 // out_tokens[b] = lowest index of the maximum bf16 logit of row b; positions[b] += 1.
-__global__ void __launch_bounds__(1024) k_bd_argmax_advance(const bf16* __restrict__ logits, int vocab, int* __restrict__ out_tokens,
+__global__ void __launch_bounds__(1024) k_bd_argmax_advance(const bf16* logits, int vocab, int* __restrict__ out_tokens,
                                                             int* __restrict__ positions, float* __restrict__ logits_f32) {
     pdl_trigger();   // the next grid may be scheduled already (it waits the same way)
     pdl_wait();      // launched with programmatic stream serialisation: the preceding grid has completed
@@ -532,9 +530,8 @@ __global__ void __launch_bounds__(1024) k_bd_argmax_advance(const bf16* __restri
     const bf16* row = logits + (size_t)b * vocab;
     unsigned long long best = 0ull;
     // 16-byte loads, eight logits each (the vocabulary is a multiple of 128 and rows are 16-byte aligned)
-    const uint4* row4 = reinterpret_cast<const uint4*>(row);
     for (int i4 = tid; i4 < vocab / 8; i4 += blockDim.x) {
-        const uint4 q = row4[i4];
+        const uint4 q = ld_cg_u4(row + i4 * 8);
         const uint32_t wds[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
@@ -557,7 +554,7 @@ __global__ void __launch_bounds__(1024) k_bd_argmax_advance(const bf16* __restri
     if (tid == 0) {
         for (int i = 1; i < (int)(blockDim.x >> 5); ++i) best = s_best[i] > best ? s_best[i] : best;
         out_tokens[b] = (int)(0xffffffffu - (uint32_t)(best & 0xffffffffull));
-        positions[b] += 1;
+        positions[b] = ld_cg_i32(positions + b) + 1;
     }
 }
 

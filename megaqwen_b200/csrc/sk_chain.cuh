@@ -338,12 +338,12 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
 }
 
 // h[s,:] = embed[ids[s],:] and the row's sums of squares
-__global__ void __launch_bounds__(128) k_sk_embed(const int* __restrict__ ids, const bf16* __restrict__ embed, bf16* __restrict__ h, float* __restrict__ ssq,
+__global__ void __launch_bounds__(128) k_sk_embed(const int* ids, const bf16* __restrict__ embed, bf16* __restrict__ h, float* __restrict__ ssq,
                                                   int vocab, unsigned int* status) {
     pdl_wait();
     pdl_trigger();   // only now: the kernels behind may read cache rows of earlier steps ahead of their own waits
     const int s = blockIdx.x, tid = threadIdx.x;
-    int tok = ids[s];
+    int tok = ld_cg_i32(ids + s);
     if (tok < 0 || tok >= vocab) {
         if (tid == 0) atomicOr(status, MQ_STATUS_BAD_TOKEN);
         tok = min(max(tok, 0), vocab - 1);

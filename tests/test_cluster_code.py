@@ -1,5 +1,6 @@
-"""Device code, read on the host: no kernel touches another CTA's shared memory before a barrier over the whole cluster has
-said that all of its CTAs run."""
+"""Device code, read on the host.  No kernel touches another CTA's shared memory before a barrier over the whole cluster has
+said that all of its CTAs run.  And what a kernel of a chain reads behind its wait, because the kernel before it wrote it, is not
+declared as data that nobody writes: such a load may be moved ahead of the wait."""
 import os
 import re
 
@@ -51,3 +52,19 @@ def test_the_rule_sees_the_kernels():
     seen = {f for n in ("sk_chain.cuh", "tc_gemm2.cuh", "hy_attention.cu") for f, body in bodies(open(os.path.join(CSRC, n)).read()) if ACCESS.search(body)}
     assert {"k_sk", "k_gemm2", "merge_pieces"} <= seen
     assert first_access_without_barrier("x(); if (a) { cluster_wait(); } st_cluster_f32(p, v);")
+
+
+WEIGHTS = {"embed", "audio", "w", "wq", "wk", "cos", "sin"}            # written by nothing on the stream
+
+
+@pytest.mark.parametrize("name", ["prefill.cu", "sk_chain.cuh", "mma_attention.cuh", "tc_attention.cuh", "tc_gemm.cuh", "tc_gemm2.cuh"])
+def test_only_weights_are_read_only(name):
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+    found = 0
+    for m in re.finditer(r"\b(\w+)\(([^;{}]*)\) \{\n", text):
+        if text[text.rfind("\n", 0, m.start()) + 1].isspace() or re.search(r"\bk_kv_quantize", m.group(0)):      # the latter is launched without overlap
+            continue
+        for p in re.finditer(r"const \w+\* __restrict__ (\w+)", m.group(0)):
+            found += 1
+            assert p.group(1) in WEIGHTS, (m.group(1), p.group(1))
+    assert found or name != "prefill.cu"
