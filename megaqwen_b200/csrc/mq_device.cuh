@@ -277,17 +277,19 @@ __device__ __forceinline__ float dot_slice(const bf16* wrow_smem, const float (&
     return a0 + a1;
 }
 
+__device__ __forceinline__ float slice_square_sum(const float (&x)[32]) {
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) ss = fmaf(x[i], x[i], ss);
+    return warp_sum(ss);
+}
 // RMSNorm of a 1024-wide bf16 vector held as a register slice per lane (every
 // warp holds the whole vector): x <- bf16(w * bf16(x * rsqrt(mean(x^2) + eps))).
 __device__ __forceinline__ void rmsnorm_slice(float (&x)[32], const bf16* w, int lane) {
     uint4 wu[4];   // requested before the row sum, used after it
 #pragma unroll
     for (int j = 0; j < 4; ++j) wu[j] = *reinterpret_cast<const uint4*>(w + j * 256 + lane * 8);
-    float ss = 0.f;
-#pragma unroll
-    for (int i = 0; i < 32; ++i) ss = fmaf(x[i], x[i], ss);
-    ss = warp_sum(ss);
-    const float r = 1.0f / sqrtf(ss * (1.0f / H) + RMS_EPS);
+    const float r = 1.0f / sqrtf(slice_square_sum(x) * (1.0f / H) + RMS_EPS);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const uint4 u = wu[j];

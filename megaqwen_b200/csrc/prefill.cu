@@ -963,7 +963,7 @@ static int decode_batch_impl(const MqModel* model, const MqBatchBuffers* bb, con
         SkArgs a = sk_args(model, B, h, bb->partials, (bf16*)bb->k_cache, (bf16*)bb->v_cache, status);
         a.pos_rows = bb->positions;
         a.seq_stride = seq_stride;
-        launch_pdl(k_sk_embed, dim3(B), dim3(128), 0, stream, in_tokens, (const bf16*)model->embed, h, a.ssq, model->vocab_size, status);
+        launch_pdl(k_sk_embed, dim3(B), dim3(32), 0, stream, in_tokens, (const bf16*)model->embed, h, a.ssq, model->vocab_size, status);
         for (int l = 0; l < model->num_layers; ++l) {
             rc = sk_qkv(model, l, a, qkv, stream);
             if (rc) return rc;
@@ -971,7 +971,7 @@ static int decode_batch_impl(const MqModel* model, const MqBatchBuffers* bb, con
             rc = sk_rest(model, l, a, attn, act, stream);
             if (rc) return rc;
         }
-        launch_pdl(k_pf_rmsnorm, dim3((B + 7) / 8), dim3(256), 0, stream, h, (const bf16*)model->final_norm, x, B);
+        launch_pdl(k_sk_norm, dim3((B + 7) / 8), dim3(256), 0, stream, h, a.ssq, (const bf16*)model->final_norm, x, B);
     } else {
     launch_pdl(k_pf_embed, dim3(B), dim3(128), 0, stream, in_tokens, (const bf16*)model->embed, h, model->vocab_size, status,
                (const bf16*)nullptr, 0, 0);

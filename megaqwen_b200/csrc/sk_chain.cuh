@@ -13,7 +13,7 @@
 // added are those of the eight kernels.  Prompts of as many rows do not come here: their sums over K are not split.
 //
 // RMSNorm: the kernel that finishes a row of the residual stream leaves the row's sum of squares of its 128 columns
-// in ssq[row][8]; the next linear adds the eight, normalises its K slice of the rows itself and writes it
+// in ssq[row][8]; the next linear adds the eight, first to last, normalises its K slice of the rows itself and writes it
 // as the swizzled operand tile that TMA would have written.
 #pragma once
 
@@ -60,6 +60,8 @@ struct SkArgs {
     int drop = -1;                 // test hook: block drop % 16 of rank drop / 16 of every cluster is never requested
 };
 
+// of the eight sums of a row, first to last
+__device__ __forceinline__ float row_square_sum(const float4& a, const float4& b) { return ((((((a.x + a.y) + a.z) + a.w) + b.x) + b.y) + b.z) + b.w; }
 // products of two pairs of bf16, each rounded once
 __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
     uint32_t r;
@@ -189,14 +191,11 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
         }
     }
     if (NORM) {
-        // row -> 1 / rms from the eight partial sums, eight lanes a row
-        static_assert(SK_SSQ == 8, "eight lanes a row");
-        constexpr int RI = (MPAD * 8 + SK_THREADS - 1) / SK_THREADS;
-        float p[RI];
-#pragma unroll
-        for (int i = 0; i < RI; ++i) {
-            const int e = tid + i * SK_THREADS;
-            p[i] = e < a.M * 8 ? ld_cg_f32(a.ssq + e) : 0.f;
+        static_assert(MPAD <= SK_THREADS, "a thread a row");
+        float4 p[2] = {};
+        if (tid < a.M) {
+            p[0] = __ldcg(reinterpret_cast<const float4*>(a.ssq + tid * SK_SSQ));
+            p[1] = __ldcg(reinterpret_cast<const float4*>(a.ssq + tid * SK_SSQ) + 1);
         }
         // this CTA's K slice of the rows: a warp takes a row at a time, a lane 16 bytes of it; all requested before the first is used
         constexpr int CI = MPAD / 8;
@@ -206,15 +205,7 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
             const int row = warp + 8 * i;
             v[i] = row < a.M ? ld_cg_u4(a.h + (size_t)row * H + kb0 * SK_BK + lane * 8) : make_uint4(0u, 0u, 0u, 0u);
         }
-#pragma unroll
-        for (int i = 0; i < RI; ++i) {
-            const int e = tid + i * SK_THREADS;
-            float s = p[i];
-            s += __shfl_xor_sync(0xffffffffu, s, 1);
-            s += __shfl_xor_sync(0xffffffffu, s, 2);
-            s += __shfl_xor_sync(0xffffffffu, s, 4);
-            if ((e & 7) == 0 && e < MPAD * 8) inv[e >> 3] = 1.0f / sqrtf(s * (1.0f / H) + RMS_EPS);
-        }
+        if (tid < a.M) inv[tid] = 1.0f / sqrtf(row_square_sum(p[0], p[1]) * (1.0f / H) + RMS_EPS);
         __syncthreads();
         // 128-byte swizzle: 16-byte chunk j of row r of a k-block stands at chunk j ^ (r & 7), and r & 7 is this warp's number
         uint8_t* dst = xs + (lane >> 3) * Cfg::X_BYTES + warp * 128 + (((lane & 7) ^ warp) << 4);
@@ -337,27 +328,48 @@ k_sk(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMa
     if (warp == 1) tmem_dealloc(tmem, TM_COLS);
 }
 
-// h[s,:] = embed[ids[s],:] and the row's sums of squares
-__global__ void __launch_bounds__(128) k_sk_embed(const int* ids, const bf16* __restrict__ embed, bf16* __restrict__ h, float* __restrict__ ssq,
-                                                  int vocab, unsigned int* status) {
+// h[s,:] = embed[ids[s],:], one warp per row.  The row's sum of squares stands in the first of its eight places, in the order in which
+// rmsnorm_slice adds it.
+__global__ void __launch_bounds__(32) k_sk_embed(const int* ids, const bf16* __restrict__ embed, bf16* __restrict__ h, float* __restrict__ ssq,
+                                                 int vocab, unsigned int* status) {
     pdl_wait();
     pdl_trigger();   // only now: the kernels behind may read cache rows of earlier steps ahead of their own waits
-    const int s = blockIdx.x, tid = threadIdx.x;
+    const int s = blockIdx.x, lane = threadIdx.x;
     int tok = ld_cg_i32(ids + s);
     if (tok < 0 || tok >= vocab) {
-        if (tid == 0) atomicOr(status, MQ_STATUS_BAD_TOKEN);
+        if (lane == 0) atomicOr(status, MQ_STATUS_BAD_TOKEN);
         tok = min(max(tok, 0), vocab - 1);
     }
-    const uint4 u = __ldg(reinterpret_cast<const uint4*>(embed + (size_t)tok * H) + tid);
-    reinterpret_cast<uint4*>(h + (size_t)s * H)[tid] = u;
-    const uint32_t x[4] = {u.x, u.y, u.z, u.w};
-    float ss = 0.f;
+    float v[32];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) ss = fmaf(bf_lo(x[q]), bf_lo(x[q]), fmaf(bf_hi(x[q]), bf_hi(x[q]), ss));
-    // 16 threads hold the 128 columns of one partial sum
+    for (int j = 0; j < 4; ++j) {
+        const uint4 u = __ldg(reinterpret_cast<const uint4*>(embed + (size_t)tok * H + j * 256) + lane);
+        *(reinterpret_cast<uint4*>(h + (size_t)s * H + j * 256) + lane) = u;
+        v[j * 8 + 0] = bf_lo(u.x); v[j * 8 + 1] = bf_hi(u.x); v[j * 8 + 2] = bf_lo(u.y); v[j * 8 + 3] = bf_hi(u.y);
+        v[j * 8 + 4] = bf_lo(u.z); v[j * 8 + 5] = bf_hi(u.z); v[j * 8 + 6] = bf_lo(u.w); v[j * 8 + 7] = bf_hi(u.w);
+    }
+    const float ss = slice_square_sum(v);
+    if (lane < SK_SSQ) ssq[(size_t)s * SK_SSQ + lane] = lane == 0 ? ss : 0.f;
+}
+
+// x[s,:] = norm of h[s,:] behind the last layer, one warp per row
+__global__ void __launch_bounds__(256) k_sk_norm(const bf16* h, const float* ssq, const bf16* __restrict__ w, bf16* __restrict__ x, int rows) {
+    pdl_trigger();
+    const int lane = threadIdx.x & 31, s = blockIdx.x * 8 + (threadIdx.x >> 5);
+    uint4 g[4];
 #pragma unroll
-    for (int o = 1; o < 16; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if ((tid & 15) == 0) ssq[(size_t)s * SK_SSQ + (tid >> 4)] = ss;
+    for (int j = 0; j < 4; ++j) g[j] = __ldg(reinterpret_cast<const uint4*>(w + j * 256) + lane);
+    pdl_wait();
+    if (s >= rows) return;
+    const float4 p0 = __ldcg(reinterpret_cast<const float4*>(ssq + (size_t)s * SK_SSQ)), p1 = __ldcg(reinterpret_cast<const float4*>(ssq + (size_t)s * SK_SSQ) + 1);
+    const float r = 1.0f / sqrtf(row_square_sum(p0, p1) * (1.0f / H) + RMS_EPS);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint4 u = ld_cg_u4(h + (size_t)s * H + j * 256 + lane * 8);
+        *(reinterpret_cast<uint4*>(x + (size_t)s * H + j * 256) + lane) =
+            make_uint4(mul_bf16x2(g[j].x, pack_bf16x2(bf_lo(u.x) * r, bf_hi(u.x) * r)), mul_bf16x2(g[j].y, pack_bf16x2(bf_lo(u.y) * r, bf_hi(u.y) * r)),
+                       mul_bf16x2(g[j].z, pack_bf16x2(bf_lo(u.z) * r, bf_hi(u.z) * r)), mul_bf16x2(g[j].w, pack_bf16x2(bf_lo(u.w) * r, bf_hi(u.w) * r)));
+    }
 }
 
 // ---------------------------------------------------------------- host side
