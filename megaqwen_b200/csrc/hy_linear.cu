@@ -143,11 +143,12 @@ static long long tile_cost(TileShape s, int M, int N, int kblocks, int split, in
 static TileShape pick_tile(int M, int N, int kblocks, int max_split, int* split) {
     static const TileShape shapes[] = {{256, 2}, {128, 2}, {256, 1}, {128, 1}, {64, 1}, {256, 0}};
     TileShape best = shapes[3];
+    const int sms = sm_count();
     long long cost = -1;
     for (const TileShape& s : shapes)
         for (int z = 1; z <= max_split && z * 4 <= kblocks + 3; z *= 2) {
             // every plane is written and read back once: 8 bytes per element over the memory of the whole device
-            const long long c = tile_cost(s, M, N, kblocks, z, sm_count()) + (long long)(z - 1) * ((long long)M * N / 500 + 1500);
+            const long long c = tile_cost(s, M, N, kblocks, z, sms) + (long long)(z - 1) * ((long long)M * N / 500 + 1500);
             if (cost < 0 || c < cost) { cost = c; best = s; *split = z; }
         }
     return best;
