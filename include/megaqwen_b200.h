@@ -269,8 +269,8 @@ typedef struct MqBatchBuffers {
     MqPrefillBuffers act;     /* activation buffers, max_tokens >= batch        */
     unsigned int* status;
     int batch;
-    float* partials;          /* optional fp32 scratch of the split-K path (batch <= 64):        */
-    size_t partials_bytes;    /* at least 4 * batch * 6144 * 4 bytes; NULL = 128-row tile GEMMs  */
+    float* partials;          /* optional 16-byte aligned fp32 scratch of the cluster chain      */
+    size_t partials_bytes;    /* (batch <= 64), 32 bytes per sequence; NULL = 128-row tile GEMMs */
     float* attn_parts;        /* optional fp32 scratch that lets several CTAs share the keys of  */
     size_t attn_parts_bytes;  /* one (sequence, kv head): at least batch * 8 * 4 * 2 * 130 * 4   */
     unsigned int* attn_tickets; /* bytes, with u32 [batch * 8] counters zeroed ONCE by the caller; */
@@ -304,13 +304,16 @@ int mq_launch_prefill_packed(const MqModel* model, const MqBatchBuffers* bb, con
 int mq_launch_decode_batch_kv8(const MqModel* model, const MqBatchBuffers* bb, const MqKvFp8* kv8,
                                const int* in_tokens, int* out_tokens, float* logits_f32, void* stream);
 
-/* Kernels one step launches on the tile-GEMM path (batch > 64); the cluster chain of smaller batches launches five per
- * layer and four more. */
+/* Kernels one step launches on the tile-GEMM path (batch > 64). */
 int mq_decode_batch_launch_count(int num_layers);
+/* Kernels one mq_launch_decode_batch call with these buffers launches. */
+int mq_decode_batch_launches(int num_layers, const MqBatchBuffers* bb);
 
-/* Number of kernels one mq_launch_prefill call launches, at most (fewer for few rows, where O and down split K,
- * and where the epilogue of q|k|v fills the caches). */
+/* Kernels of one mq_launch_prefill call on the path of most row counts below 512. */
 int mq_prefill_launch_count(int num_layers);
+/* Kernels one mq_launch_prefill call of `rows` rows launches, or (packed) one mq_launch_prefill_packed call of as many rows
+ * in all; max_tokens: that of the MqPrefillBuffers. */
+int mq_prefill_launches(int num_layers, int rows, int max_tokens, int packed);
 
 /* C[M,N] = A[M,K] * B[N,K]^T (+ R), bf16 row-major, fp32 accumulation, on the
  * tcgen05 path; N a multiple of 128, K a multiple of 64, lda/ldc multiples of

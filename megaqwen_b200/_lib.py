@@ -95,7 +95,9 @@ SIGNATURES = {
                                        C.c_void_p, C.c_void_p, C.c_int, C.c_void_p]),
     "mq_launch_decode_batch_kv8": (C.c_int, [C.POINTER(MqModel), C.POINTER(MqBatchBuffers), C.POINTER(MqKvFp8), C.c_void_p, C.c_void_p,
                                              C.c_void_p, C.c_void_p]),
+    "mq_decode_batch_launches": (C.c_int, [C.c_int, C.POINTER(MqBatchBuffers)]),
     "mq_prefill_launch_count": (C.c_int, [C.c_int]),
+    "mq_prefill_launches": (C.c_int, [C.c_int] * 4),
     "mq_launch_gemm_bf16": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int,
                                       C.c_int, C.c_void_p, C.c_void_p]),
     "mq_debug_gemm_drop_load": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int,

@@ -60,7 +60,7 @@ class MegakernelBatchDecoder:
             self._counters = torch.zeros(16, dtype=i32, device=dev)
             self._slot = torch.zeros(1, dtype=torch.int64, device=dev)
             self._tok_a = torch.zeros(B, dtype=i32, device=dev)
-            self._partials = torch.empty(4 * min(B, 64) * 2 * _INTER, dtype=torch.float32, device=dev)
+            self._partials = torch.empty(8 * min(B, 64), dtype=torch.float32, device=dev)      # row sums of the cluster chain
             # split-KV scratch of the batched attention: (m, l, acc[128]) per (sequence, kv head, part, head) and one ticket per item
             self._attn_parts = torch.empty(B * _NKV * 4 * 2 * (_D + 2), dtype=torch.float32, device=dev)
             self._attn_tickets = torch.zeros(B * _NKV, dtype=i32, device=dev)
@@ -93,10 +93,7 @@ class MegakernelBatchDecoder:
                               _ptr(self._attn_tickets) if self.use_split_kv else None)
 
     def _step_launches(self, batch: int) -> int:
-        """Kernels of one step: up to 64 rows the cluster chain of five per layer."""
-        if batch <= 64 and self.use_splitk:
-            return 1 + 5 * self.num_layers_ + 3
-        return self._lib.mq_decode_batch_launch_count(self.num_layers_)
+        return self._lib.mq_decode_batch_launches(self.num_layers_, C.byref(self._bb(batch)))
 
     def check_status(self) -> None:
         st = int(self._scalars[1].item())
@@ -160,7 +157,7 @@ class MegakernelBatchDecoder:
         rc = self._lib.mq_launch_prefill_packed(C.byref(self._model), C.byref(bb), *offs, total, int(tile_seq.numel()),
                                                 _ptr(out) + 4 * b0, self._stream())
         _lib.check(rc, "mq_launch_prefill_packed")
-        self.launches += 1 + 8 * self.num_layers_ + 4
+        self.launches += self._lib.mq_prefill_launches(self.num_layers_, total, self._pf.max_tokens, 1)
         self._keep = dev_t     # the launch reads the tables asynchronously
 
     def prefill_batch(self, prompts) -> torch.Tensor:
@@ -205,7 +202,7 @@ class MegakernelBatchDecoder:
                 rc = self._lib.mq_launch_prefill(C.byref(self._model), C.byref(dbuf), C.byref(self._pf), _ptr(dev_ids), n, 0,
                                                  _ptr(out) + 4 * b, None, self._stream())
                 _lib.check(rc, "mq_launch_prefill")
-                self.launches += self._lib.mq_prefill_launch_count(self.num_layers_)
+                self.launches += self._lib.mq_prefill_launches(self.num_layers_, n, self._pf.max_tokens, 0)
                 lens.append(n)
             self._positions[: len(prompts)].copy_(torch.tensor(lens, dtype=torch.int32), non_blocking=False)
         self.batch_ = len(prompts)

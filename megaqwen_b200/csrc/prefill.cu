@@ -562,7 +562,6 @@ __global__ void __launch_bounds__(1024) k_bd_argmax_advance(const bf16* logits, 
 
 using namespace mq;
 
-// kernels of one prefill (at most: the split-K path needs one norm kernel fewer per layer after the first)
 extern "C" int mq_prefill_launch_count(int num_layers) { return 1 + num_layers * 8 + 2; }
 
 // C[M,N] = A[M,K] * B[N,K]^T on the tcgen05 path (bf16 in/out, fp32 accumulate);
@@ -655,8 +654,9 @@ extern "C" int mq_debug_chain_drop_load(const MqModel* model, const MqBatchBuffe
 //   gate|up 16.0 / 18.5  30.0 / 19.9  30.3 / 25.3  59.1 / 42.4   242 / 148
 //   o       14.5 / 18.3  14.7 / 18.5  14.6 / 19.4  29.2 / 22.2   131 / 76
 //   down    19.3 / 23.9  20.0 / 24.3  20.1 / 25.1  39.4 / 27.9   155 / 85
-// Below, tiles are as wide as leaves one round of CTAs.  Prompt of 2 / 23 / 128 / 256 / 384 / 640 / 900 / 1024 rows with 128-wide tiles
+// Below, tiles are as wide as leaves one round of CTAs on the 148 SMs of the device (the counts beside the rules).  Prompt of 2 / 23 / 128 / 256 / 384 / 640 / 900 / 1024 rows with 128-wide tiles
 // everywhere: 1.76 / 1.82 / 2.00 / 2.03 / 2.10 / 2.22 / 2.72 / 2.41 ms, now 1.67 / 1.71 / 1.86 / 1.93 / 2.00 / 2.12 / 2.30 / 2.33.
+static bool heads_on_pairs(int rows) { return (rows > 512 && rows <= 1024) || rows > 9 * 128; }
 static int pf_qkv(const MqModel* model, int l, const bf16* x, bf16* qkv, int rows, Heads hd, unsigned int* status, cudaStream_t stream) {
     const MqLayerWeights& w = model->layers[l];
     const bf16 *q = (const bf16*)w.q_proj, *k = (const bf16*)w.k_proj, *v = (const bf16*)w.v_proj;
@@ -665,7 +665,7 @@ static int pf_qkv(const MqModel* model, int l, const bf16* x, bf16* qkv, int row
     // q | k | v in one launch: column tiles from three weight matrices.  The pairs' epilogue, which runs under the next tile's products,
     // norms, rotates and fills the caches as well, so they pay from 513 rows on (16 column tiles x 3 row tiles) but for the five row tiles that
     // make 80 on 74 pairs (1100 rows 2.66, on pairs 2.90 ms).
-    if ((rows > 512 && rows <= 1024) || rows > 9 * 128) return launch_gemm2<256, EPI_HEADS>(x, H, q, k, qkv, nullptr, rows, QKV, H, QKV, status, stream, v, QSZ, KVSZ, 1, true, hd);
+    if (heads_on_pairs(rows)) return launch_gemm2<256, EPI_HEADS>(x, H, q, k, qkv, nullptr, rows, QKV, H, QKV, status, stream, v, QSZ, KVSZ, 1, true, hd);
     const int rc = rows > 1024 ? launch_gemm<256, EPI_STORE, 1>(x, H, q, k, qkv, nullptr, rows, QKV, H, QKV, status, stream, v, QSZ, KVSZ)
                  : rows > 256  ? launch_gemm<128, EPI_STORE>(x, H, q, k, qkv, nullptr, rows, QKV, H, QKV, status, stream, v, QSZ, KVSZ)
                                : launch_gemm<64, EPI_STORE>(x, H, q, k, qkv, nullptr, rows, QKV, H, QKV, status, stream, v, QSZ, KVSZ);
@@ -687,6 +687,23 @@ static int pf_add(const bf16* A, int K, const bf16* W, bf16* h, int rows, unsign
     if (rows > 18 * 128) return launch_gemm2<256, EPI_RESID>(A, K, W, nullptr, h, h, rows, H, K, H, status, stream);
     if (rows > 1024) return launch_gemm<128, EPI_RESID>(A, K, W, nullptr, h, h, rows, H, K, H, status, stream);
     return launch_gemm<64, EPI_RESID>(A, K, W, nullptr, h, h, rows, H, K, H, status, stream);
+}
+
+// Between 512 and 1024 rows the N = 1024 projections (O, down) split K over two CTAs per 128 x 128 tile:
+// 64-wide tiles re-read the A operand sixteen times and are bound by L2 traffic.  The fp32 planes land in
+// the qkv buffer (free after attention; 2 x rows x 1024 floats fill it exactly) and one kernel adds them to the
+// residual stream and applies the RMSNorm that follows (the next layer's input norm after the down projection).
+// Above 1024 and up to 2048 rows the same with 128 x 256 tiles (N = 256 instructions, half the A traffic per FLOP).
+// Below, sums over K stay whole.
+static bool planes_of_k(int rows, int max_tokens) {
+    return rows >= 512 && rows <= 2048 && (size_t)max_tokens * QKV * sizeof(bf16) >= (size_t)2 * rows * H * sizeof(float);
+}
+
+// Kernels of one pass over `rows` rows.  A layer: q|k|v, heads (unless the product's epilogue does them), attention, O, norm, gate|up, down
+// and a norm, ahead of q|k|v or, with planes, behind down (and once ahead of the first layer).  Around: embedding, last row, LM head;
+// packed: embedding, last rows, norm, LM head, arg-max.
+extern "C" int mq_prefill_launches(int num_layers, int rows, int max_tokens, int packed) {
+    return num_layers * (heads_on_pairs(rows) ? 7 : 8) + (packed ? 5 : planes_of_k(rows, max_tokens) ? 4 : 3);
 }
 
 extern "C" int mq_launch_prefill(const MqModel* model, const MqDecodeBuffers* dbuf, const MqPrefillBuffers* pb, const int* ids,
@@ -740,13 +757,7 @@ static int prefill_impl(const MqModel* model, const MqDecodeBuffers* dbuf, const
     int rc;
     launch_pdl(k_pf_embed, dim3(S), dim3(128), 0, stream, ids, (const bf16*)model->embed, h, model->vocab_size, status, audio,
                audio_start, audio_len);
-    // Between 512 and 1024 rows the N = 1024 projections (O, down) split K over two CTAs per 128 x 128 tile:
-    // 64-wide tiles re-read the A operand sixteen times and are bound by L2 traffic.  The fp32 planes land in
-    // the qkv buffer (free after attention; 2 x S x 1024 floats fill it exactly) and one kernel adds them to the
-    // residual stream and applies the RMSNorm that follows (the next layer's input norm after the down projection).
-    // Above 1024 and up to 2048 rows the same with 128 x 256 tiles (N = 256 instructions, half the A traffic per FLOP).
-    // Below, sums over K stay whole.
-    const bool splitk = S >= 512 && S <= 2048 && (size_t)pb->max_tokens * QKV * sizeof(bf16) >= (size_t)2 * S * H * sizeof(float);
+    const bool splitk = planes_of_k(S, pb->max_tokens);
     const bool wide = splitk && S > 1024;
     float* part = reinterpret_cast<float*>(qkv);
     Heads heads = {};
@@ -864,8 +875,14 @@ extern "C" int mq_launch_prefill_packed(const MqModel* model, const MqBatchBuffe
     return (int)cudaGetLastError();
 }
 
-// kernels of one step on the tile-GEMM path (batch > 64); the cluster chain of smaller batches launches five per layer
 extern "C" int mq_decode_batch_launch_count(int num_layers) { return 1 + num_layers * 10 + 3; }
+// up to 64 rows: the cluster chain (sk_chain.cuh), its row sums in the caller's scratch; above, tile GEMMs
+static bool on_chain(int batch, const float* partials, size_t bytes) {
+    return batch <= SK_MAX_ROWS && partials != nullptr && bytes >= (size_t)batch * SK_SSQ * sizeof(float);
+}
+extern "C" int mq_decode_batch_launches(int num_layers, const MqBatchBuffers* bb) {
+    return on_chain(bb->batch, bb->partials, bb->partials_bytes) ? num_layers * 5 + 4 : mq_decode_batch_launch_count(num_layers);
+}
 
 // How a batched attention launch is shaped for `items` = 8 x batch (sequence, kv head) pairs.  Up to one
 // item per SM: twelve-warp CTAs, the keys of every item split over up to four CTAs while those still fit one
@@ -957,9 +974,7 @@ static int decode_batch_impl(const MqModel* model, const MqBatchBuffers* bb, con
     const bool can_split = bb->attn_parts != nullptr && bb->attn_tickets != nullptr &&
                            bb->attn_parts_bytes >= (size_t)B * NKV * BD_MAX_PARTS * 2 * BD_PART * sizeof(float);
     const BdShape shape = bd_shape(B * NKV, sm_count[dev_now], can_split);
-    // up to 64 rows: the cluster chain (sk_chain.cuh), its row sums in the caller's scratch; above, tile GEMMs
-    const bool skinny = B <= SK_MAX_ROWS && bb->partials != nullptr && bb->partials_bytes >= (size_t)B * SK_SSQ * sizeof(float);
-    if (skinny) {
+    if (on_chain(B, bb->partials, bb->partials_bytes)) {
         SkArgs a = sk_args(model, B, h, bb->partials, (bf16*)bb->k_cache, (bf16*)bb->v_cache, status);
         a.pos_rows = bb->positions;
         a.seq_stride = seq_stride;

@@ -314,7 +314,7 @@ class MegakernelDecoder(DecodeEngine):
                 rc = self._lib.mq_launch_prefill(C.byref(self._model), C.byref(self._buf), C.byref(self._pf), _ptr(dev_ids), n,
                                                  self.position_, _ptr(self._scalars), logits_ptr, self._stream())
             _lib.check(rc, "mq_launch_prefill")
-            self.launches += self._lib.mq_prefill_launch_count(self.num_layers_)
+            self.launches += self._lib.mq_prefill_launches(self.num_layers_, n, self._pf.max_tokens, 0)
             self.position_ += n
             self._kv8_ready = 0        # the prefill wrote bf16 rows only (bindings_prefill.cpp:831)
             tok, status = self._scalars[:2].tolist()
