@@ -1,5 +1,5 @@
-"""The cluster chain of few rows (prompts of up to 128 tokens, batches of up to 64) at the edges of its operand widths
-(16, 32, 64, 128 rows) and of the shares that the CTAs of a cluster finish, against the restatement."""
+"""Few rows against the restatement: prompts of up to 128 tokens, and the cluster chain of a batch's steps at the edges of its
+operand widths (16, 32, 64 rows) and of the shares that the CTAs of a cluster finish."""
 import pytest
 import torch
 

@@ -41,8 +41,8 @@ def test_whole_prompt_against_portions(args, rows):
 
 @pytest.mark.parametrize("rows", [129, 256, 257, 384, 385, 511, 512, 513, 768, 769, 1000, 1024])
 def test_prompt_against_portions_of_few_rows(args, rows):
-    """Every choice of tiles up to 1024 rows against portions of at most 128 rows, which take the cluster chain: other sums, so
-    two bf16 computations that differ by their roundings, two spacings at [4, 8) at most."""
+    """Every choice of tiles up to 1024 rows against portions of at most 128 rows, whose attention walks its keys in other tiles: two
+    bf16 computations that differ by their roundings, two spacings at [4, 8) at most."""
     from megaqwen_b200.decoder import MegakernelDecoder
     dec = MegakernelDecoder(*args, MAX_SEQ, MAX_SEQ)
     p = random_prompt(QWEN3_TINY, rows, 33, rows)
