@@ -331,7 +331,7 @@ int mq_launch_gemm_bf16(const void* A, int lda, const void* B, void* C, const vo
 int mq_debug_gemm_drop_load(const void* A, int lda, const void* B, void* C, int M, int N, int K, int ldc,
                             unsigned int* status, void* stream, int drop_kb);
 
-/* The same for the GEMM on pairs of SMs, C = A B^T + R with N a multiple of 256: a pair of SMs computes several 256 x 256 tiles one
+/* The same for the GEMM on pairs of SMs, C = A B^T + R with N a multiple of 256 and B complete before the call: a pair of SMs computes several 256 x 256 tiles one
  * after the other (pair p the tiles p, p + pairs, ..); drop_kb counts the k-blocks of one pair over all of its tiles, and
  * the tiles before the one that lacks a block are stored.  drop_kb = -1: nothing is left out. */
 int mq_debug_gemm_pair_drop_load(const void* A, int lda, const void* B, void* C, const void* R, int M, int N, int K, int ldc,

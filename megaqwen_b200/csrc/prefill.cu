@@ -587,14 +587,14 @@ extern "C" int mq_debug_gemm_drop_load(const void* A, int lda, const void* B, vo
                                        nullptr, 0, 0, 1, drop_kb, false);
 }
 
-// The same for the GEMM on pairs of SMs (N a multiple of 256), whose pairs walk several tiles each: drop_kb counts a pair's k-blocks over
-// all of its tiles, and the tiles before the one that lacks a block are stored.  drop_kb = -1: the GEMM as it is.
+// The same for the GEMM on pairs of SMs (N a multiple of 256; B complete before the call), whose pairs walk several tiles each: drop_kb counts
+// a pair's k-blocks over all of its tiles, and the tiles before the one that lacks a block are stored.  drop_kb = -1: the GEMM as it is.
 extern "C" int mq_debug_gemm_pair_drop_load(const void* A, int lda, const void* B, void* C, const void* R, int M, int N, int K, int ldc,
                                             unsigned int* status, void* stream, int drop_kb) {
     if (!A || !B || !C || !R || !status || M <= 0 || N <= 0 || K <= 0 || drop_kb < -1) return MQ_ERR_BAD_ARG;
     if (lda % 8 != 0 || ldc % 8 != 0) return MQ_ERR_ALIGNMENT;
     return launch_gemm2<256, EPI_RESID>((const bf16*)A, lda, (const bf16*)B, nullptr, (bf16*)C, (const bf16*)R, M, N, K, ldc, status, (cudaStream_t)stream,
-                                        nullptr, 0, 0, 1, false, NoSink(), drop_kb);
+                                        nullptr, 0, 0, 1, true, NoSink(), drop_kb);
 }
 
 static int prefill_impl(const MqModel* model, const MqDecodeBuffers* dbuf, const MqPrefillBuffers* pb, const int* ids,

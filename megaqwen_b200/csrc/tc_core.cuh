@@ -123,10 +123,11 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128(const void* tile, uint32_
 // Bounded wait that does not look at the sticky status word: used while a CTA drains after one of its
 // waits has expired (copies already issued must land, MMAs already issued must finish, before the CTA
 // hands back its shared and tensor memory).  About 1 ms.
+constexpr long long DRAIN_LIMIT_CYCLES = 2000000LL;
 __device__ __forceinline__ bool mbar_wait_drain(uint64_t* bar, uint32_t parity) {
     const long long t0 = clock64();
     while (!mbar_try_wait(bar, parity))
-        if (clock64() - t0 > 2000000LL) return false;
+        if (clock64() - t0 > DRAIN_LIMIT_CYCLES) return false;
     return true;
 }
 

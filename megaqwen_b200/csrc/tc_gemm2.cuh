@@ -167,10 +167,9 @@ k_gemm2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtenso
         }
     };
 
-    int c = 0;                                // k-blocks requested so far, over all tiles (producer)
+    int c = 0, npre = 0;                      // k-blocks requested so far, over all tiles, and those whose B tile is requested early (producer)
     if (warp == 0) {
         if (lane == 0) {
-            int npre = 0;
             if (a.early_b && first < tiles) { // the first tile's weights, ring permitting, before the preceding grid has finished
                 int tm, tn, z, kb0, nk;
                 place(first, tm, tn, z, kb0, nk);
@@ -345,13 +344,12 @@ k_gemm2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtenso
     }
     __syncthreads();
     // After an expired wait (which the other CTA of the pair then runs into as well): copies that were requested still land.  The leader
-    // waits for the last of every stage; the other CTA, whose copies report to the leader's barriers, for as long as the leader waits
-    // for one of them at most.
+    // waits for the last of every stage, with a limit; the other CTA, whose copies report to the leader's barriers, for as long as that limit.
     if (*aborted && tid == 0) {
         if (leader)
-            for (int s = 0; s < ST && s < c; ++s) mbar_wait_drain(&full[s], (uint32_t)(((c - 1 - s) / ST)) & 1u);
+            for (int s = 0; s < ST && s < max(c, npre); ++s) mbar_wait_drain(&full[s], c > s ? (uint32_t)((c - 1 - s) / ST) & 1u : 0u);
         else
-            mbar_wait_drain(drained, 0);      // nothing arrives there
+            for (const long long t0 = clock64(); clock64() - t0 < DRAIN_LIMIT_CYCLES;) {}
     }
     __syncwarp();
     cluster_sync_all();                       // both CTAs' copies, products and remote arrivals are done

@@ -56,9 +56,9 @@ def test_gemm_on_pairs(m, k, drop, whole):
     a, b, r = (torch.randn(s, generator=g, device="cuda", dtype=torch.bfloat16) for s in ((m, k), (256, k), (m, 256)))
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
 
-    def run(drop_kb):
+    def run(drop_kb, before=0):
         c = torch.full((m, 256), 7.0, dtype=torch.bfloat16, device="cuda")
-        status.zero_()
+        status.fill_(before)
         rc = lib.mq_debug_gemm_pair_drop_load(a.data_ptr(), k, b.data_ptr(), c.data_ptr(), r.data_ptr(), m, 256, k, 256, status.data_ptr(),
                                               torch.cuda.current_stream().cuda_stream, drop_kb)
         _lib.check(rc, "mq_debug_gemm_pair_drop_load")
@@ -76,3 +76,7 @@ def test_gemm_on_pairs(m, k, drop, whole):
         assert torch.equal(c[:256 * whole], right[:256 * whole]) and bool((c[256 * whole:] == 7.0).all())
     again, st = run(-1)
     assert st == 0 and torch.equal(again, right)
+    for _ in range(20):                                # behind an expired wait every wait gives up after a few polls: whatever is in flight ends first
+        run(-1, _lib.MQ_STATUS_WAIT_TIMEOUT)
+        again, st = run(-1)
+        assert st == 0 and torch.equal(again, right)
